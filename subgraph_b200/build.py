@@ -23,10 +23,12 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"] + ARCH
 CXX_FLAGS = ["-std=c++17", "-O3", "-fPIC", "-Wall", "-Wno-unused-function"]
 
-HOST_SOURCES = ["host/graph_io.cpp", "host/plan.cpp", "capi.cpp"]
+HOST_SOURCES = ["host/graph_io.cpp", "host/plan.cpp", "capi.cpp", "engine/rooted_plan.cpp"]
 CUDA_SOURCES = ["engine/kernels.cu", "engine/blocked.cu", "engine/blocked_a.cu", "engine/blocked_b.cu",
                 "engine/blocked_c.cu", "engine/blocked_d.cu", "engine/blocked_e.cu", "engine/engine.cu", "engine/batch.cu", "engine/noalloc.cu",
-                "engine/input_gpu.cu"]
+                "engine/input_gpu.cu",
+                "engine/rooted.cu", "engine/rooted_gather_f32.cu", "engine/rooted_gather_f64.cu", "engine/rooted_ema.cu", "engine/rooted_ema_a.cu", "engine/rooted_ema_b.cu",
+                "engine/rooted_ema_c.cu", "engine/rooted_ema_d.cu", "engine/rooted_ema_e.cu"]
 
 
 def _cuda_home() -> str:

@@ -12,6 +12,7 @@
 
 #include "blk_sched.hpp"
 #include "kernels.cuh"
+#include "rooted.hpp"
 #include "tile.cuh"
 
 namespace sg {
@@ -111,6 +112,17 @@ struct Workspace {
     int32_t *tile_ticket = nullptr;    // fused kernels' tile counters, one per concurrent stream
     size_t tile_ticket_bytes = 0;
     uint64_t generation = 0;   // bumped whenever a buffer above is re-allocated
+    // rooted rows: aggregates, neighbour counts and their scaled copy, counters
+    void *agg = nullptr;
+    size_t agg_bytes = 0;
+    void *cnt = nullptr;
+    size_t cnt_bytes = 0;
+    void *scnt = nullptr;
+    size_t scnt_bytes = 0;
+    double *root = nullptr;            // root values of a main that is not one-hot
+    size_t root_bytes = 0;
+    int32_t *rticket = nullptr;
+    size_t rticket_bytes = 0;
 };
 
 struct DevicePlanTables {
@@ -183,6 +195,13 @@ std::mutex g_state_mu;
 // one copy per (device, plan) serves every graph (a graph uploaded per call
 // finds them ready); release_plan_tables frees them with the plan.
 std::map<std::pair<int, uint64_t>, DevicePlanTables> g_plan_tables;   // guarded by g_state_mu
+
+// The rooted rows' plan and tables, kept and released like the tables above.
+struct RootedEntry {
+    rt::RootedPlan plan[2];   // FP32, FP64
+    rt::RootedTables tab;
+};
+std::map<std::pair<int, uint64_t>, RootedEntry> g_rooted;   // guarded by g_state_mu
 
 void free_plan_tables(DevicePlanTables &t)
 {
@@ -361,6 +380,19 @@ bool build_blocks(const IndexView &st, std::vector<int32_t> &rows, int &nblocks,
     }
     return true;
 }
+
+}  // namespace
+
+bool rt::rooted_blocks(int k, int n, int pm, std::vector<int32_t> &rows, int &nblocks, int &shape)
+{
+    int L = 0, S = 0;
+    std::vector<int32_t> c2c, ms, as;
+    index_tables(k, n, pm, L, S, c2c, ms, as);
+    const IndexView iv{k, n, pm, L, S, c2c.data(), ms.data(), as.data()};
+    return build_blocks(iv, rows, nblocks, shape);
+}
+
+namespace {
 
 // the `size` colors (ascending) of the color set with colex rank r
 void colex_unrank(int size, int64_t r, int *out)
@@ -631,7 +663,7 @@ DeviceGraph::~DeviceGraph()
             Workspace &w = it->second.ws;
             for (void *p : {w.arena, (void *)w.colors, (void *)w.partial, (void *)w.raw, (void *)w.windows, w.hub_partial,
                             (void *)w.chunk_start, (void *)w.root_vertex, (void *)w.adjc, (void *)w.orig_buf,
-                            (void *)w.hub_ticket, (void *)w.tile_ticket})
+                            (void *)w.hub_ticket, (void *)w.tile_ticket, w.agg, w.cnt, w.scnt, (void *)w.root, (void *)w.rticket})
                 if (p) cudaFreeAsync(p, stream);
             for (auto &kv : it->second.batches) free_batch(kv.second, stream);
             for (cudaStream_t js : it->second.streams) {
@@ -704,6 +736,13 @@ static void color_tables(int blocks, std::vector<uint32_t> &jump, std::vector<ui
     coef = g_coef;
 }
 
+// vertices of degree d or more: a prefix of the degree-descending order
+static int32_t degree_prefix(const DeviceGraph &g, int32_t d)
+{
+    return (int32_t)(std::partition_point(g.h_degree.begin(), g.h_degree.end(), [&](int32_t x) { return x >= d; }) -
+                     g.h_degree.begin());
+}
+
 // The common tail of every graph upload: the degree order (on the device),
 // the relabelled adjacency (k_remap from the original-order device arrays,
 // which this frees) and the coloring jump-ahead tables.
@@ -719,14 +758,16 @@ Status graph_finish(DeviceGraph &gr, int32_t *d_old_off, int32_t *d_old_adj)
     SG_CK(cudaMallocAsync(&g->d_iperm, sizeof(int32_t) * std::max<int32_t>(V, 1), st));
     SG_CKS(degree_order(V, d_old_off, g->d_iperm, g->d_perm, g->d_off, g->h_degree, st));
     g->max_degree = V ? g->h_degree[0] : 0;
+    g->V1 = degree_prefix(*g, 1);
+    g->V2 = degree_prefix(*g, 2);
     int32_t *d_bad = nullptr;
-    const int32_t none = INT32_MAX;
-    int32_t bad = none;
-    SG_CK(cudaMallocAsync(&d_bad, sizeof(int32_t), st));
-    SG_CK(cudaMemcpyAsync(d_bad, &none, sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    launch_remap(V, d_old_off, d_old_adj, g->d_off, g->d_iperm, g->d_perm, g->d_adj, d_bad, st);
+    const int32_t none[2] = {INT32_MAX, 0};
+    int32_t bad[2] = {INT32_MAX, 0};
+    SG_CK(cudaMallocAsync(&d_bad, sizeof none, st));
+    SG_CK(cudaMemcpyAsync(d_bad, none, sizeof none, cudaMemcpyHostToDevice, st));
+    launch_remap(V, nnz, d_old_off, d_old_adj, g->d_off, g->d_iperm, g->d_perm, g->d_adj, g->V2, d_bad, st);
     SG_CK(cudaGetLastError());
-    SG_CK(cudaMemcpyAsync(&bad, d_bad, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    SG_CK(cudaMemcpyAsync(bad, d_bad, sizeof bad, cudaMemcpyDeviceToHost, st));
     cudaFreeAsync(d_bad, st);
     // coloring jump-ahead tables
     g->color_blocks = (V + kColorBlock - 1) / kColorBlock;
@@ -739,7 +780,10 @@ Status graph_finish(DeviceGraph &gr, int32_t *d_old_off, int32_t *d_old_adj)
     cudaFreeAsync(d_old_off, st);
     cudaFreeAsync(d_old_adj, st);
     SG_CK(cudaStreamSynchronize(st));
-    if (bad != none) return Status{1, "neighbour id out of range at entry " + std::to_string(bad)};
+    if (bad[0] != none[0]) return Status{1, "neighbour id out of range at entry " + std::to_string(bad[0])};
+    // the rows of the vertices of degree 1 are left out only where each such
+    // vertex is listed by its own neighbour alone
+    if (bad[1]) g->V2 = g->V1;
     return Status::ok();
 }
 
@@ -756,6 +800,16 @@ void release_plan_tables(uint64_t uid)
         cudaSetDevice(it->first.first);
         free_plan_tables(it->second);   // cudaFree waits for the device's work
         it = g_plan_tables.erase(it);
+    }
+    for (auto it = g_rooted.begin(); it != g_rooted.end();) {
+        if (it->first.second != uid) {
+            ++it;
+            continue;
+        }
+        if (prev < 0) cudaGetDevice(&prev);
+        cudaSetDevice(it->first.first);
+        cudaFree(it->second.tab.mem);
+        it = g_rooted.erase(it);
     }
     if (prev >= 0) cudaSetDevice(prev);
 }
@@ -809,6 +863,7 @@ struct RunCtx {
     bool use_adjc = false;   // one coloring at a time per slot: neighbour ids carry their colors
     void *hub_region = nullptr;  // this context's hub partial rows (job streams), else the workspace's
     int ticket = 0;              // its hub item and tile counters (job streams: the stream's)
+    const RootedEntry *re = nullptr;   // the rooted rows, when the call takes them
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> fused_ev, hub_ev;
     std::vector<std::pair<int, double>> fused_sub;   // per fused launch: sub, compulsory bytes
     double fused_alg_bytes = 0, fused_gather_bytes = 0;
@@ -1147,6 +1202,9 @@ Status run_stage(RunCtx &c, int slot, int s, double *root_vertex, cudaStream_t s
             SG_CK(cudaEventCreate(&e1));
             float best = 1e30f;
             for (auto cand : candidate_shapes(d, c.fp64)) {
+                // the root's tile size is the untuned one: it decides the order of
+                // the FP64 sum, which is the same in every form and run
+                if (d.is_root && cand.tile_v != d.tile_v) continue;
                 StageDesc dc = d;
                 if (!set_shape(dc, c.fp64, cand)) continue;
                 FusedConfig cc = cfg;
@@ -1596,6 +1654,397 @@ Status count_batched(RunCtx &c, const CountOptions &o, double *raw, CountStats *
     return Status::ok();
 }
 
+
+// ---------------------------------------------------------------------------
+// Rooted rows (rooted.hpp): the plain form and the job streams.
+// ---------------------------------------------------------------------------
+// The calls that take them: the pruned modes with no form switched off (the
+// switches select the general path's forms), shapes that fit the kernels.
+bool takes_rooted(const CountOptions &o) { return (o.mode == kModeReference || o.mode == kModeFP64) && o.blocked && o.rooted && o.flat; }
+
+// What the general path does untuned for sub s: its tile size (the root's sums
+// equal it bit for bit), and whether its products are fused multiply-adds (the
+// packed form, which it takes outside exact mode where no block schedule has
+// the shape).  False: the step does not fit its tiles.
+bool general_form(const Plan &p, int s, bool fp64, int &tile_v, bool &fused)
+{
+    const SubTemplate &r = p.subs[s], &m = p.subs[r.main], &a = p.subs[r.aux];
+    StageDesc d{};
+    d.V = 1;
+    d.k = p.k;
+    d.nb = 1;
+    d.is_root = s == 0;
+    d.main_leaf = m.size == 1;
+    d.aux_leaf = a.size == 1;
+    d.L_s = r.L;
+    d.S = r.S;
+    d.L_m = d.main_cols = m.L;
+    d.L_a = a.L;
+    d.aux_cols = d.aux_leaf ? p.k : a.L;
+    static const uint32_t some = 0;
+    if (s != 0 && m.size > 1 && !fp64) d.aoff = d.moff = &some;
+    FusedConfig cfg;
+    const bool ok = plan_fused(d, fp64, 148, cfg);
+    tile_v = ok ? d.tile_v : 32;
+    fused = ok && d.packed == 1 && !blk::shape_id(r.size, m.size) &&
+            (a.size < 2 || !blk::shape_id(r.size - 1, m.size - 1));
+    return ok;
+}
+
+Status rooted_entry(DeviceGraph &g, const Plan &p, const RootedEntry *&out)
+{
+    const std::pair<int, uint64_t> key{g.device, p.uid};
+    {
+        std::lock_guard<std::mutex> lk(g_state_mu);
+        auto it = g_rooted.find(key);
+        if (it != g_rooted.end()) {
+            out = &it->second;
+            return Status::ok();
+        }
+    }
+    RootedEntry e;
+    e.plan[0] = rt::make_rooted_plan(p, false);
+    e.plan[1] = rt::make_rooted_plan(p, true);
+    for (int f = 0; f < 2; ++f)
+        for (rt::Step &q : e.plan[f].steps)   // templates too large for the general path's tiles stay refused there
+            if (!general_form(p, q.s, f == 1, q.root_tile, q.fused)) e.plan[f].ok = false;
+    if (e.plan[0].ok || e.plan[1].ok) {
+        const cudaError_t ce = rt::upload_rooted_tables(p, e.plan[0], e.tab, g.stream);
+        if (ce != cudaSuccess) {
+            cudaFree(e.tab.mem);
+            return Status{ce == cudaErrorMemoryAllocation ? 2 : 3, std::string("rooted tables: ") + cudaGetErrorString(ce)};
+        }
+    }
+    std::lock_guard<std::mutex> lk(g_state_mu);
+    auto ins = g_rooted.try_emplace(key, std::move(e));
+    if (!ins.second) cudaFree(e.tab.mem);   // another thread made them first
+    out = &ins.first->second;
+    return Status::ok();
+}
+
+// The buffers of one coloring in flight.
+struct RootedSlot {
+    char *arena, *agg, *cnt, *scnt;
+    int32_t *adjd;
+    uint8_t *color;
+    double *partial, *root;
+    int32_t *ticket;
+};
+constexpr int kRootedStreams = 4;
+// counters of a step: the column blocks' chunks, the hub items last; a slot
+// has them for every step of a template (at most 15)
+constexpr int kStepTickets = 64, kRootedTickets = 16 * kStepTickets;
+
+// Per-slot bytes of a plan whose tables have `rows` rows.
+struct RootedSizes {
+    size_t arena = 0, agg = 0, cnt = 0, scnt = 0, adjd = 0;
+    size_t all() const { return arena + agg + cnt + scnt + adjd; }
+    void cover(const RootedSizes &o)
+    {
+        arena = std::max(arena, o.arena);
+        agg = std::max(agg, o.agg);
+        cnt = std::max(cnt, o.cnt);
+        scnt = std::max(scnt, o.scnt);
+        adjd = std::max(adjd, o.adjd);
+    }
+};
+RootedSizes rooted_sizes(const DeviceGraph &g, const rt::RootedPlan &rp, int32_t rows, size_t es)
+{
+    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    RootedSizes z;
+    z.arena = up((size_t)rp.arena_units * rows * es);
+    z.agg = up(std::max((size_t)rp.agg_pitch * rows, (size_t)g.V1) * es);
+    z.cnt = up((size_t)rp.cnt_pitch * g.V1 * es);
+    z.scnt = rp.need_scaled ? z.cnt : 0;
+    z.adjd = rp.need_edges ? up(4 * (size_t)g.nnz) : 0;
+    return z;
+}
+
+Status rooted_reserve(DeviceGraph &g, Workspace &w, const RootedSizes &z, int slots, int ncolorings, std::vector<RootedSlot> &out)
+{
+    cudaStream_t st = g.stream;
+    const size_t V = (size_t)g.V, n = (size_t)slots;
+    auto some = [](size_t x) { return std::max<size_t>(16, x); };
+    SG_CKS(grow(&w.arena, &w.arena_bytes, some(z.arena * n), st));
+    SG_CKS(grow(&w.agg, &w.agg_bytes, some(z.agg * n), st));
+    SG_CKS(grow(&w.cnt, &w.cnt_bytes, some(z.cnt * n), st));
+    SG_CKS(grow(&w.scnt, &w.scnt_bytes, some(z.scnt * n), st));
+    SG_CKS(growT(&w.adjc, &w.adjc_bytes, some(z.adjd * n), st));
+    SG_CKS(growT(&w.colors, &w.colors_bytes, some(V * n), st));
+    SG_CKS(growT(&w.partial, &w.partial_bytes, 8 * (V / 8 + 2) * n, st));
+    SG_CKS(growT(&w.root, &w.root_bytes, 8 * (size_t)std::max(g.V1, 1) * n, st));
+    SG_CKS(growT(&w.rticket, &w.rticket_bytes, 4 * kRootedTickets * n, st));
+    SG_CKS(growT(&w.raw, &w.raw_bytes, 8 * (size_t)std::max(ncolorings, 1), st));
+    SG_CKS(growT(&w.windows, &w.windows_bytes, 4 * 31 * (size_t)std::max(ncolorings, 1), st));
+    out.clear();
+    for (size_t i = 0; i < n; ++i)
+        out.push_back({(char *)w.arena + z.arena * i, (char *)w.agg + z.agg * i, (char *)w.cnt + z.cnt * i,
+                       (char *)w.scnt + z.scnt * i, w.adjc + z.adjd / 4 * i, w.colors + V * i,
+                       w.partial + (V / 8 + 2) * i, w.root + (size_t)std::max(g.V1, 1) * i, w.rticket + kRootedTickets * i});
+    return Status::ok();
+}
+
+const void *rooted_table(const RunCtx &c, const rt::RootedPlan &rp, const RootedSlot &w, int32_t rows, int sub)
+{
+    const rt::SubTable &t = rp.tab[sub];
+    if (t.kind == 1) return w.cnt;
+    if (t.kind == 2) return w.scnt;
+    return w.arena + (size_t)t.off * rows * c.es;
+}
+
+// Vertices of more neighbours than this are a gather's hubs (a CTA's chain of
+// adds each) and do not share a warp's work.  Wide rows: a warp of a full SM
+// takes about 560 cycles a neighbour, and no list should outlast the work of
+// all (nnz neighbours at about 50 cycles over 148 SMs).  Narrow rows: about
+// 150 cycles a neighbour against the longest hub's 12.
+int hub_deg(const DeviceGraph &g, int nA)
+{
+    if (nA <= 1) return 256;
+    const int64_t d = nA > 64 ? g.nnz / 4096 : g.max_degree / 12;
+    return (int)std::min<int64_t>(8192, std::max<int64_t>(256, d));
+}
+
+// One coloring (window `coloring`) on stream st: tables of `rows` rows, the
+// steps of the subs >= upto, with the root step its raw count.
+Status run_rooted(RunCtx &c, const RootedSlot &w, int32_t rows, int coloring, double *raw_out, double *root_vertex, int upto,
+                  cudaStream_t st)
+{
+    DeviceGraph &g = c.g;
+    const rt::RootedPlan &rp = c.re->plan[c.fp64];
+    const rt::RootedTables &tab = c.re->tab;
+    ColorArgs ca{};
+    ca.V = g.V;
+    ca.k = c.p.k;
+    ca.nblocks = g.color_blocks;
+    ca.jump = g.d_jump;
+    ca.coef = g.d_coef;
+    ca.window = c.gs.ws.windows + 31 * (size_t)coloring;
+    ca.perm = g.d_perm;
+    ca.color = w.color;
+    ca.color_stride = g.V;
+    ca.vertex_stride = 1;
+    launch_color(ca, 1, st);
+    rt::EdgeArgs ea{};
+    ea.V1 = g.V1;
+    ea.lim = rows;
+    ea.k = c.p.k;
+    ea.hubs = degree_prefix(g, 1025);
+    ea.off = g.d_off;
+    ea.adj = g.d_adj;
+    ea.color = w.color;
+    ea.adjd = rp.need_edges ? w.adjd : nullptr;
+    ea.cnt = w.cnt;
+    ea.scnt = rp.need_scaled ? w.scnt : nullptr;
+    ea.cnt_pitch = rp.cnt_pitch;
+    rt::launch_edges(ea, std::max(ea.hubs, degree_prefix(g, 32)), c.fp64, st);
+    c.launches += 2;
+    SG_CK(cudaGetLastError());
+    SG_CK(cudaMemsetAsync(w.ticket, 0, 4 * kStepTickets * rp.steps.size(), st));
+    int root_n = 0;
+    for (size_t i = 0; i < rp.steps.size(); ++i) {
+        const rt::Step &q = rp.steps[i];
+        if (q.s < upto) break;
+        const SubTemplate &sub = c.p.subs[q.s];
+        const bool root = q.s == 0;
+        const int32_t V = root && q.main_leaf ? g.V1 : rows;
+        const void *agg = w.cnt;
+        int agg_pitch = rp.cnt_pitch;
+        if (c.profile) {
+            SG_CKS(ev_pair(c.fused_ev));
+            SG_CK(cudaEventRecord(c.fused_ev.back().first, st));
+        }
+        if (!q.aux_leaf) {
+            rt::GatherArgs ga{};
+            ga.k = c.p.k;
+            ga.nA = q.nA;
+            ga.nR = (int)binom(c.p.k - 1, q.m - 1);
+            ga.V = V;
+            ga.pitch = rp.tab[sub.aux].pitch;
+            ga.off = g.d_off;
+            ga.adjd = w.adjd;
+            ga.aux = rooted_table(c, rp, w, rows, sub.aux);
+            ga.idx = tab.idx[i];
+            const rt::ColumnOrder &co = rt::columns(c.p.k, q.m);
+            ga.members = co.members;
+            ga.slots = co.slots;
+            std::copy(co.start, co.start + rt::kMaxMembers + 1, ga.start);
+            if (root && q.main_leaf) ga.out = w.agg, ga.out_pitch = 1;
+            else if (q.main_leaf) ga.out = const_cast<void *>(rooted_table(c, rp, w, rows, q.s)), ga.out_pitch = rp.tab[q.s].pitch;
+            else ga.out = w.agg, ga.out_pitch = rp.agg_pitch;
+            ga.hubs = std::min(V, degree_prefix(g, hub_deg(g, q.nA) + 1));
+            ga.map = rt::make_chunks(g.h_degree, ga.hubs, V, 512, 32 / rt::gather_lanes(ga), 32);
+            ga.ticket = w.ticket + kStepTickets * i;
+            ga.hub_ticket = ga.ticket + kStepTickets - 1;
+            c.launches += rt::launch_gather(ga, c.fp64, g.sm_count, st);
+            agg = ga.out;
+            agg_pitch = ga.out_pitch;
+        }
+        if (!q.main_leaf) {
+            rt::EmaArgs ma{};
+            ma.k = c.p.k;
+            ma.V = V;
+            ma.nA = q.nA;
+            ma.nM = q.nM;
+            ma.nO = q.nO;
+            ma.S = tab.S[i];
+            ma.agg = agg;
+            ma.agg_pitch = agg_pitch;
+            ma.main = rooted_table(c, rp, w, rows, sub.main);
+            ma.main_pitch = rp.tab[sub.main].pitch;
+            ma.is_root = root;
+            ma.fused = q.fused && !c.exact;
+            if (!root) {
+                ma.out = const_cast<void *>(rooted_table(c, rp, w, rows, q.s));
+                ma.out_pitch = rp.tab[q.s].pitch;
+                ma.perm_o = tab.perm[q.n - 1];
+            }
+            ma.color = w.color;
+            ma.perm_a = tab.perm[q.m];
+            ma.perm_m = tab.perm[q.pm - 1];
+            ma.split = tab.split[i];
+            ma.split_stride = tab.split_stride[i];
+            ma.blk = tab.blk[i];
+            ma.blk_shape = tab.blk_shape[i];
+            ma.blk_nblocks = tab.blk_nblocks[i];
+            ma.root_value = w.root;
+            rt::launch_ema(ma, c.fp64, st);
+            c.launches += V > 0;
+        }
+        if (root) {
+            rt::RootArgs ra{};
+            ra.V1 = V;
+            ra.pitch = q.main_leaf ? agg_pitch : 1;
+            ra.tile_v = q.root_tile;
+            ra.val = q.main_leaf ? agg : w.root;
+            ra.root_partial = w.partial;
+            ra.root_vertex = root_vertex;
+            root_n = rt::launch_root_tiles(ra, c.fp64 || !q.main_leaf, st);
+            c.launches += root_n > 0;
+        }
+        if (c.profile) {
+            SG_CK(cudaEventRecord(c.fused_ev.back().second, st));
+            // compulsory traffic: aux and main rows read once (one-hot children: the
+            // colors), the result's written once, the adjacency read once
+            const double la = q.aux_leaf ? 1.0 : (double)binom(c.p.k - 1, q.m - 1), lm = q.main_leaf ? 1.0 : (double)q.nM;
+            const double alg = (double)c.es * V * (la + lm + (root ? 0.0 : (double)q.nO)) + 4.0 * (g.V1 + 1.0 + (double)g.nnz);
+            c.fused_alg_bytes += alg;
+            c.fused_sub.push_back({q.s, alg});
+            c.fused_gather_bytes += (double)c.es * (double)g.nnz * (q.aux_leaf ? 0.25 : la);
+        }
+        SG_CK(cudaGetLastError());
+    }
+    if (upto == 0) {
+        launch_root_reduce(w.partial, root_n, c.mode == kModeReference ? 1.0e12 : 1.0, raw_out, st);
+        c.launches += 1;
+        SG_CK(cudaGetLastError());
+    }
+    return Status::ok();
+}
+
+Status upload_seeds(DeviceGraph &g, Workspace &w, const std::vector<uint32_t> &seeds)
+{
+    std::vector<uint32_t> win(seeds.size() * 31);
+    for (size_t i = 0; i < seeds.size(); ++i) glibc_window(seeds[i], &win[i * 31]);
+    // pageable source: the call returns once it has been read
+    SG_CK(cudaMemcpyAsync(w.windows, win.data(), win.size() * 4, cudaMemcpyHostToDevice, g.stream));
+    return Status::ok();
+}
+
+// Streams joined: `st` waits for the first n job streams.
+void join_streams(GraphState &gs, int n, cudaStream_t st)
+{
+    for (int s = 0; s < n; ++s) {
+        cudaEvent_t e;
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) {
+            cudaEventRecord(e, gs.streams[s]);
+            cudaStreamWaitEvent(st, e, 0);
+            cudaEventDestroy(e);
+        }
+    }
+}
+
+Status make_streams(GraphState &gs, int n)
+{
+    while ((int)gs.streams.size() < n) {
+        cudaStream_t js;
+        SG_CK(cudaStreamCreateWithFlags(&js, cudaStreamNonBlocking));
+        gs.streams.push_back(js);
+    }
+    return Status::ok();
+}
+
+// Slots for up to `want` colorings in flight that fit the free memory.
+Status rooted_admit(const DeviceGraph &g, const Workspace &w, const RootedSizes &z, int want, int &slots)
+{
+    slots = std::max(1, want);
+    if (slots == 1) return Status::ok();
+    // buffers that are there already need no answer from the driver
+    const size_t n = (size_t)slots;
+    if (w.arena_bytes >= z.arena * n && w.agg_bytes >= z.agg * n && w.cnt_bytes >= z.cnt * n && w.scnt_bytes >= z.scnt * n &&
+        w.adjc_bytes >= z.adjd * n && w.colors_bytes >= (size_t)g.V * n)
+        return Status::ok();
+    size_t free_b = 0, total_b = 0;
+    SG_CK(cudaMemGetInfo(&free_b, &total_b));
+    const size_t per = z.all() + (size_t)g.V + 8 * ((size_t)g.V / 8 + 2) + 8 * (size_t)g.V1;
+    const size_t have = w.arena_bytes + w.agg_bytes + w.cnt_bytes + w.scnt_bytes + w.adjc_bytes;
+    while (slots > 1 && per * (size_t)slots > (size_t)((double)(free_b + have) * 0.85)) --slots;
+    return Status::ok();
+}
+
+Status count_rooted(RunCtx &c, const CountOptions &o, double *raw, CountStats *stats)
+{
+    DeviceGraph &g = c.g;
+    Workspace &w = c.gs.ws;
+    cudaStream_t st = g.stream;
+    const RootedSizes z = rooted_sizes(g, c.re->plan[c.fp64], g.V2, c.es);
+    // several colorings in flight: the chains of one's hubs run beside the
+    // others' work (profiled launches one after another)
+    int S = 1;
+    const int most = o.batch > 0 ? std::min(o.batch, kRootedStreams) : kRootedStreams;
+    SG_CKS(rooted_admit(g, w, z, c.profile ? 1 : std::min(o.n_colorings, most), S));
+    std::vector<RootedSlot> slot;
+    SG_CKS(rooted_reserve(g, w, z, S, o.n_colorings, slot));
+    std::vector<uint32_t> seeds(o.n_colorings);
+    for (int i = 0; i < o.n_colorings; ++i) seeds[i] = o.seed_base + (uint32_t)i;
+    SG_CKS(upload_seeds(g, w, seeds));
+    if (S > 1) SG_CKS(make_streams(c.gs, S));
+    cudaEvent_t e0, e1;
+    SG_CK(cudaEventCreate(&e0));
+    SG_CK(cudaEventCreate(&e1));
+    SG_CK(cudaEventRecord(e0, st));
+    if (S > 1)
+        for (int s = 0; s < S; ++s) SG_CK(cudaStreamWaitEvent(c.gs.streams[s], e0, 0));
+    Status status = Status::ok();
+    for (int i = 0; i < o.n_colorings && !status.code; ++i)
+        status = run_rooted(c, slot[i % S], g.V2, i, w.raw + i, nullptr, 0, S > 1 ? c.gs.streams[i % S] : st);
+    if (S > 1) join_streams(c.gs, S, st);
+    if (status.code) {
+        cudaStreamSynchronize(st);
+        return status;
+    }
+    SG_CK(cudaEventRecord(e1, st));
+    SG_CK(cudaMemcpyAsync(raw, w.raw, sizeof(double) * o.n_colorings, cudaMemcpyDeviceToHost, st));
+    SG_CK(cudaStreamSynchronize(st));
+    float ms = 0;
+    cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    if (stats) {
+        stats->device_ms = ms;
+        stats->kernel_launches = c.launches;
+        stats->table_bytes = (int64_t)((z.arena + z.agg + z.cnt + z.scnt) * S);
+        stats->fused_launches = (int64_t)c.fused_ev.size();
+        top_stage(c, stats);
+        stats->fused_ms = ev_sum(c.fused_ev);
+        stats->hub_ms = ev_sum(c.hub_ev);
+        stats->fused_alg_bytes = c.fused_alg_bytes;
+        stats->fused_gather_bytes = c.fused_gather_bytes;
+    }
+    ev_sum(c.fused_ev);
+    ev_sum(c.hub_ev);
+    return Status::ok();
+}
+
 }  // namespace
 
 // Interleaved groups: colorings per launch of each stage.  Every candidate
@@ -1728,6 +2177,12 @@ Status count(DeviceGraph &g, const Plan &p, const CountOptions &o, double *raw, 
     SG_CK(cudaSetDevice(g.device));
     GraphState &gs = state_of(g);
     RunCtx c{g, p, gs, nullptr, o.mode == kModeFP64, (size_t)(o.mode == kModeFP64 ? 8 : 4), 0, {}, 0, 0, o.mode, 0};
+    c.profile = o.profile != 0;
+    c.exact = o.exact != 0;
+    if (takes_rooted(o) && !(o.batch > 0 && o.persistent)) {
+        SG_CKS(rooted_entry(g, p, c.re));
+        if (c.re->plan[c.fp64].ok) return count_rooted(c, o, raw, stats);
+    }
     SG_CKS(make_ctx_tables(g, p, gs, c.tab));
     c.exact = o.exact != 0;
     // hubs in exact order (the per-tile sums) on the plain and grouped forms;
@@ -1847,6 +2302,7 @@ Status debug_sub_table(DeviceGraph &g, const Plan &p, uint32_t seed, int mode, i
     std::vector<int32_t> perm(g.V);
     if (g.V) SG_CK(cudaMemcpy(perm.data(), g.d_perm, 4 * (size_t)g.V, cudaMemcpyDeviceToHost));
     const size_t V = (size_t)g.V;
+    if (g.V >= (1 << 28)) return Status{1, "counting supports graphs of fewer than 2^28 vertices"};
     if (sub.size == 1) {
         std::vector<int32_t> col(V);
         SG_CKS(debug_colors(g, p.k, seed, col.data()));
@@ -1856,6 +2312,46 @@ Status debug_sub_table(DeviceGraph &g, const Plan &p, uint32_t seed, int mode, i
                 if (c.fp64) ((double *)out)[cc * V + v] = val;
                 else ((float *)out)[cc * V + v] = (float)val;
             }
+        return Status::ok();
+    }
+    c.exact = true;   // the reference's operation order
+    if (mode == kModeReference || mode == kModeFP64) SG_CKS(rooted_entry(g, p, c.re));
+    if (c.re && c.re->plan[c.fp64].ok) {
+        // every vertex's row (the counting calls leave out the rows nobody reads)
+        const rt::RootedPlan &rp = c.re->plan[c.fp64];
+        std::vector<RootedSlot> slot;
+        SG_CKS(rooted_reserve(g, gs.ws, rooted_sizes(g, rp, g.V1, c.es), 1, 1, slot));
+        SG_CKS(upload_seeds(g, gs.ws, {seed}));
+        SG_CKS(run_rooted(c, slot[0], g.V1, 0, nullptr, nullptr, s, g.stream));
+        SG_CK(cudaStreamSynchronize(g.stream));
+        const int P = rp.tab[s].pitch, k = p.k;
+        std::vector<char> rows((size_t)g.V1 * P * c.es);
+        std::vector<uint8_t> color(V);
+        if (g.V1) SG_CK(cudaMemcpy(rows.data(), rooted_table(c, rp, slot[0], g.V1, s), rows.size(), cudaMemcpyDeviceToHost));
+        if (V) SG_CK(cudaMemcpy(color.data(), slot[0].color, V, cudaMemcpyDeviceToHost));
+        // column of each (color, color set): the set relative to the color, -1 without it
+        std::vector<int32_t> col((size_t)k * sub.L, -1);
+        for (int b = 0; b < k; ++b)
+            for (int cc = 0; cc < sub.L; ++cc) {
+                int el[32];
+                unsigned t = 0;
+                colex_unrank(sub.size, cc, el);
+                bool holds = false;
+                for (int i = 0; i < sub.size; ++i) {
+                    if (el[i] == b) holds = true;
+                    else t |= 1u << ((el[i] - b + k) % k - 1);
+                }
+                if (holds) col[(size_t)b * sub.L + cc] = rt::columns(k, sub.size - 1).pos[t];
+            }
+        std::memset(out, 0, V * sub.L * c.es);
+        for (size_t v = 0; v < V; ++v) {
+            const int32_t i = perm[v];
+            if (i >= g.V1) continue;
+            for (int cc = 0; cc < sub.L; ++cc) {
+                const int32_t j = col[(size_t)color[i] * sub.L + cc];
+                if (j >= 0) std::memcpy((char *)out + ((size_t)cc * V + v) * c.es, rows.data() + ((size_t)i * P + j) * c.es, c.es);
+            }
+        }
         return Status::ok();
     }
     SG_CKS(run_partial(g, p, seed, mode, hub_threshold, s, c, gs));
@@ -1876,7 +2372,19 @@ Status debug_root(DeviceGraph &g, const Plan &p, uint32_t seed, int mode, int hu
     GraphState &gs = state_of(g);
     RunCtx c{g, p, gs, nullptr, mode == kModeFP64, (size_t)(mode == kModeFP64 ? 8 : 4), 0, {}, 0, 0, mode, 0};
     SG_CKS(growT(&gs.ws.root_vertex, &gs.ws.root_vertex_bytes, 8 * std::max<size_t>(1, (size_t)g.V), g.stream));
-    SG_CKS(run_partial(g, p, seed, mode, hub_threshold, 0, c, gs));
+    if (g.V >= (1 << 28)) return Status{1, "counting supports graphs of fewer than 2^28 vertices"};
+    c.exact = true;   // the reference's operation order
+    if (mode == kModeReference || mode == kModeFP64) SG_CKS(rooted_entry(g, p, c.re));
+    if (c.re && c.re->plan[c.fp64].ok) {
+        std::vector<RootedSlot> slot;
+        SG_CKS(rooted_reserve(g, gs.ws, rooted_sizes(g, c.re->plan[c.fp64], g.V2, c.es), 1, 1, slot));
+        SG_CKS(upload_seeds(g, gs.ws, {seed}));
+        SG_CK(cudaMemsetAsync(gs.ws.root_vertex, 0, 8 * std::max<size_t>(1, (size_t)g.V), g.stream));
+        SG_CKS(run_rooted(c, slot[0], g.V2, 0, gs.ws.raw, gs.ws.root_vertex, 0, g.stream));
+        SG_CK(cudaStreamSynchronize(g.stream));
+    } else {
+        SG_CKS(run_partial(g, p, seed, mode, hub_threshold, 0, c, gs));
+    }
     std::vector<double> rv(g.V);
     std::vector<int32_t> perm(g.V);
     if (g.V) {
@@ -2085,6 +2593,60 @@ Status count_jobs(DeviceGraph &g, const std::vector<const Plan *> &plans, const 
     return Status::ok();
 }
 
+// Job streams on rooted rows: job j on stream j % S, whose slot the stream's
+// jobs use one after another.
+static Status count_jobs_rooted(DeviceGraph &g, std::vector<RunCtx> &ctx, const uint32_t *seeds, const CountOptions &o,
+                                double *raw, double *job_ms, CountStats *stats)
+{
+    GraphState &gs = ctx[0].gs;
+    Workspace &w = gs.ws;
+    const int n = (int)ctx.size();
+    cudaStream_t st = g.stream;
+    RootedSizes z;
+    for (RunCtx &c : ctx) z.cover(rooted_sizes(g, c.re->plan[c.fp64], g.V2, c.es));
+    int S = 1;
+    SG_CKS(rooted_admit(g, w, z, std::min(o.batch > 0 ? o.batch : 8, n), S));
+    std::vector<RootedSlot> slot;
+    SG_CKS(rooted_reserve(g, w, z, S, n, slot));
+    SG_CKS(upload_seeds(g, w, std::vector<uint32_t>(seeds, seeds + n)));
+    SG_CKS(make_streams(gs, S));
+    std::vector<cudaEvent_t> ev_end(n, nullptr);
+    cudaEvent_t ev0;
+    SG_CK(cudaEventCreate(&ev0));
+    for (int j = 0; j < n; ++j) SG_CK(cudaEventCreate(&ev_end[j]));
+    SG_CK(cudaEventRecord(ev0, st));
+    for (int s = 0; s < S; ++s) SG_CK(cudaStreamWaitEvent(gs.streams[s], ev0, 0));
+    int64_t launches = 0;
+    Status status = Status::ok();
+    for (int j = 0; j < n && !status.code; ++j) {
+        cudaStream_t js = gs.streams[j % S];
+        status = run_rooted(ctx[j], slot[j % S], g.V2, j, w.raw + j, nullptr, 0, js);
+        if (status.code) break;
+        cudaEventRecord(ev_end[j], js);
+        launches += ctx[j].launches;
+    }
+    join_streams(gs, S, st);
+    if (!status.code) SG_CK(cudaMemcpyAsync(raw, w.raw, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+    SG_CK(cudaStreamSynchronize(st));
+    double total = 0;
+    for (int j = 0; j < n; ++j) {
+        float ms = 0;
+        if (!status.code && cudaEventElapsedTime(&ms, ev0, ev_end[j]) == cudaSuccess) {
+            if (job_ms) job_ms[j] = ms;
+            total = std::max(total, (double)ms);
+        }
+        cudaEventDestroy(ev_end[j]);
+    }
+    cudaEventDestroy(ev0);
+    if (status.code) return status;
+    if (stats) {
+        stats->device_ms = total;
+        stats->kernel_launches = launches;
+        stats->table_bytes = (int64_t)(z.all() * S);
+    }
+    return Status::ok();
+}
+
 // ---------------------------------------------------------------------------
 // Job streams, stream form: every job runs the plain form's tuned stage
 // launches (register-blocked eMA, colour-tagged neighbours, chunk masks) on
@@ -2112,6 +2674,18 @@ Status count_jobs_streams(DeviceGraph &g, const std::vector<const Plan *> &plans
     const size_t es = fp64 ? 8 : 4;
     const size_t V = (size_t)g.V;
     cudaStream_t st = g.stream;
+    if (takes_rooted(o)) {
+        bool all = true;
+        std::vector<RunCtx> rc;
+        rc.reserve(n);
+        for (int j = 0; j < n && all; ++j) {
+            rc.push_back(RunCtx{g, *plans[j], gs, nullptr, fp64, es, 0, {}, 0, 0, o.mode, 0});
+            rc.back().exact = o.exact != 0;
+            SG_CKS(rooted_entry(g, *plans[j], rc.back().re));
+            all = rc.back().re->plan[fp64].ok;
+        }
+        if (all) return count_jobs_rooted(g, rc, seeds, o, raw, job_ms, stats);
+    }
     const Hubs hubs = plan_hubs(g, o.hub_threshold, true);
     std::vector<RunCtx> ctx;
     ctx.reserve(n);

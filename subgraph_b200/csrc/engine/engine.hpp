@@ -30,6 +30,7 @@ struct DeviceGraph {
     int32_t V = 0;
     int64_t nnz = 0;
     int32_t max_degree = 0;
+    int32_t V1 = 0, V2 = 0;       // vertices of degree 1 or more; whose table rows are read (rooted.hpp)
     int32_t *d_off = nullptr;     // [V+1] internal order
     int32_t *d_adj = nullptr;     // [nnz]
     int32_t *d_perm = nullptr;    // original -> internal

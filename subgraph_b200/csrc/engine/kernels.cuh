@@ -37,9 +37,11 @@ void launch_color_adj(const int32_t *adj, int64_t nnz, const uint8_t *color, int
                       cudaStream_t st);
 // relabelled adjacency; a neighbour id outside [0, V) is not followed: the
 // first such entry's index is kept in *bad (atomicMin; the caller starts it
-// at INT32_MAX) and a 0 is written in its place
-void launch_remap(int32_t V, const int32_t *old_off, const int32_t *old_adj, const int32_t *new_off,
-                  const int32_t *iperm, const int32_t *perm, int32_t *new_adj, int32_t *bad, cudaStream_t st);
+// at INT32_MAX) and a 0 is written in its place.  bad[1] (0 at first) becomes
+// 1 when some vertex lists a neighbour of degree 1 (internal ids V2 and up)
+// that lists another vertex
+void launch_remap(int32_t V, int64_t nnz, const int32_t *old_off, const int32_t *old_adj, const int32_t *new_off,
+                  const int32_t *iperm, const int32_t *perm, int32_t *new_adj, int32_t V2, int32_t *bad, cudaStream_t st);
 
 struct FusedConfig {
     int tile_v;      // vertices per tile

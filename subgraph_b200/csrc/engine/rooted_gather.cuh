@@ -1,0 +1,628 @@
+// Device side of the rooted rows' gather (rooted.hpp), instantiated for FP32
+// and FP64 tables in rooted_gather_f32.cu and rooted_gather_f64.cu.
+#pragma once
+#include <algorithm>
+#include <atomic>
+
+#include "rooted.hpp"
+#include "tile.cuh"
+
+namespace sg {
+namespace rt {
+
+namespace {
+
+// The chunk of ticket t: its first vertex and one past its last.
+__device__ __forceinline__ bool chunk_of(const ChunkMap &m, int t, int &v0, int &v1)
+{
+    int c = 0;
+    while (c < m.n && t >= m.base[c + 1]) ++c;
+    if (c >= m.n) return false;
+    v0 = m.first[c] + (t - m.base[c]) * m.per[c];
+    v1 = min(v0 + m.per[c], m.first[c + 1]);
+    return true;
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// The gather: every vertex's sums of its neighbours' rows, at the color sets
+// without its own color, in list order.  Three parts:
+//   hubs    a CTA per (vertex, columns), the longest lists first;
+//   wide    a warp per run of vertices, R sums a lane, rows staged in shared
+//           memory by bulk copies;
+//   narrow  G lanes a vertex, R sums a lane, rows read where they lie.
+// One kernel takes the hubs first and then the wide or the narrow part, so
+// that the longest chains run beside the other vertices.
+// ---------------------------------------------------------------------------
+constexpr int kWarps = 8, kGatherThreads = 32 * kWarps;
+
+template <typename T> __device__ __forceinline__ void cp_async_elem(uint32_t dst, const void *src, uint32_t n)
+{
+    if constexpr (sizeof(T) == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+    else
+        cp_async4_zs(dst, src, n);
+}
+
+// Hubs.  A column's sum over its list is one chain of dependent adds, four
+// cycles each, so one warp does nothing but add: lane l reads column l of
+// batch after batch of neighbours from shared memory.  The other warps fill
+// the batches two ahead, 32 / GH neighbours at a time: a lane copies
+// (cp.async) the one element of the neighbour's row that its column takes, or
+// zeros.
+constexpr int kHubStages = 3;
+template <int GH> constexpr int hub_fills() { return GH == 1 ? 4 : 16; }   // a producer warp and batch
+template <typename T, int GH> constexpr size_t hub_bytes() { return (size_t)kHubStages * (kWarps - 1) * hub_fills<GH>() * 32 * sizeof(T); }
+
+template <typename T, int GH> __device__ __forceinline__ void hub_part(const GatherArgs &a, unsigned char *smem)
+{
+    constexpr int NPF = 32 / GH, PER = hub_fills<GH>(); // neighbours a fill, fills
+    constexpr int NPW = PER * NPF;                  // neighbours a producer and batch
+    constexpr int NB = (kWarps - 1) * NPW;              // neighbours a batch
+    constexpr int NWD = (NPW + 31) / 32;                // words a lane holds of them
+    T *xs = reinterpret_cast<T *>(smem);                // [kHubStages][NB][GH]
+    __shared__ uint16_t tab[16 * GH];
+    __shared__ int s_item;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lg = lane % GH, sub = lane / GH;
+    const int nblk = (a.nA + GH - 1) / GH;
+    const char *aux = reinterpret_cast<const char *>(a.aux);
+    const uint32_t row_bytes = (uint32_t)a.pitch * (uint32_t)sizeof(T);
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_item = atomicAdd(a.hub_ticket, 1);
+        __syncthreads();
+        const int v = s_item / nblk, col0 = (s_item - v * nblk) * GH;
+        if (v >= a.hubs) break;
+        for (int i = threadIdx.x; i < a.k * GH; i += kGatherThreads) {
+            const int d = i / GH, j = col0 + i % GH;
+            tab[i] = d > 0 && j < a.nA ? __ldg(a.idx + (size_t)(d - 1) * a.nA + j) : (uint16_t)0xffffu;
+        }
+        const int beg = __ldg(a.off + v), deg = __ldg(a.off + v + 1) - beg;
+        const int nbt = (deg + NB - 1) / NB;
+        __syncthreads();
+        if (warp < kWarps - 1) {
+            const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(xs) + (uint32_t)((warp * NPW * GH + lane) * sizeof(T));
+            auto words = [&](int b, uint32_t(&w)[NWD]) {
+#pragma unroll
+                for (int i = 0; i < NWD; ++i) {
+                    const int e = b * NB + warp * NPW + i * 32 + (NPW < 32 ? lane & (NPW - 1) : lane);
+                    w[i] = e < deg ? (uint32_t)__ldg(a.adjd + beg + e) : 0u;
+                }
+            };
+            auto fill = [&](int b, const uint32_t(&w)[NWD]) {
+                const uint32_t dst = dst0 + (uint32_t)((b % kHubStages) * (NB * GH * (int)sizeof(T)));
+                // the shuffles and table reads of eight fills, then their copies
+#pragma unroll
+                for (int i0 = 0; i0 < PER; i0 += 8) {
+                    constexpr int Q = PER < 8 ? PER : 8;
+                    uint32_t x[Q], c[Q];
+#pragma unroll
+                    for (int i = 0; i < Q; ++i)
+                        x[i] = GH == 1 ? w[(i0 + i) * NPF / 32] : __shfl_sync(0xffffffffu, w[(i0 + i) * NPF / 32], ((i0 + i) * NPF) % 32 + sub);
+#pragma unroll
+                    for (int i = 0; i < Q; ++i) c[i] = tab[(x[i] >> 28) * GH + lg];
+#pragma unroll
+                    for (int i = 0; i < Q; ++i) {
+                        const bool hit = c[i] != 0xffffu;
+                        const char *src = aux + (uint64_t)(x[i] & 0x0fffffffu) * row_bytes + (hit ? c[i] : 0u) * (uint32_t)sizeof(T);
+                        cp_async_elem<T>(dst + (uint32_t)((i0 + i) * 32 * sizeof(T)), src, hit ? (uint32_t)sizeof(T) : 0u);
+                    }
+                }
+            };
+            uint32_t w0[NWD], w1[NWD], w2[NWD];
+            words(0, w0);
+            words(1, w1);
+            words(2, w2);
+            fill(0, w0);
+            cp_async_commit();
+            fill(1, w1);
+            cp_async_commit();
+            for (int b = 0; b < nbt; ++b) {
+                cp_async_wait<1>();
+                __syncthreads();       // batch b is in; the adder is done with batch b - 1
+#pragma unroll
+                for (int i = 0; i < NWD; ++i) w0[i] = w2[i];
+                words(b + 3, w2);
+                fill(b + 2, w0);
+                cp_async_commit();
+            }
+            cp_async_wait<0>();
+        } else {
+            T acc = T(0);
+            for (int b = 0; b < nbt; ++b) {
+                __syncthreads();
+                const T *x = xs + (b % kHubStages) * (NB * GH) + lg;
+                const int n = min(NB, deg - b * NB);
+                int i = 0;
+                for (; i + 32 <= n; i += 32) {
+                    T y[32];
+#pragma unroll
+                    for (int u = 0; u < 32; ++u) y[u] = x[(i + u) * GH];
+#pragma unroll
+                    for (int u = 0; u < 32; ++u) acc = add_rn(acc, y[u]);
+                }
+                for (; i < n; ++i) acc = add_rn(acc, x[i * GH]);
+            }
+            if (sub == 0 && col0 + lg < a.nA) reinterpret_cast<T *>(a.out)[(size_t)v * a.out_pitch + col0 + lg] = acc;
+        }
+    }
+}
+
+// Wide.  A warp walks the neighbour entries of its vertices as one stream
+// through a ring of NBAT batches of BR rows in shared memory (cp.async, the
+// 16-byte pieces that the neighbour's color needs).  A lane then reads, for
+// each of its columns, the element the color points at (a zero behind the row
+// where it points at none).
+__device__ __forceinline__ float lds_elem(uint32_t addr, float)
+{
+    float x;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(addr));
+    return x;
+}
+__device__ __forceinline__ double lds_elem(uint32_t addr, double)
+{
+    double x;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x) : "r"(addr));
+    return x;
+}
+// base + the low or high half of w, in one instruction
+__device__ __forceinline__ uint32_t add_lo(uint32_t base, uint32_t w) { return __dp2a_lo(w, 0x0001u, base); }
+__device__ __forceinline__ uint32_t add_hi(uint32_t base, uint32_t w) { return __dp2a_lo(w, 0x0100u, base); }
+
+template <int R> __device__ __forceinline__ void add_all(float (&acc)[R], const float (&x)[R])
+{
+#pragma unroll
+    for (int r = 0; r + 1 < R; r += 2) {
+        unsigned long long a, b;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(acc[r]), "f"(acc[r + 1]));
+        asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(x[r]), "f"(x[r + 1]));
+        a = add2_rn(a, b);
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[r]), "=f"(acc[r + 1]) : "l"(a));
+    }
+    if (R & 1) acc[R - 1] = add_rn(acc[R - 1], x[R - 1]);
+}
+template <int R> __device__ __forceinline__ void add_all(double (&acc)[R], const double (&x)[R])
+{
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = add_rn(acc[r], x[r]);
+}
+
+// a += x where `second` is 0, else b += x
+__device__ __forceinline__ void add_one_of(float &a, float &b, float x, uint32_t second)
+{
+    asm("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %3, 0;\n\t@p add.rn.f32 %0, %0, %2;\n\t@!p add.rn.f32 %1, %1, %2;\n\t}"
+        : "+f"(a), "+f"(b)
+        : "f"(x), "r"(second));
+}
+__device__ __forceinline__ void add_one_of(double &a, double &b, double x, uint32_t second)
+{
+    asm("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %3, 0;\n\t@p add.rn.f64 %0, %0, %2;\n\t@!p add.rn.f64 %1, %1, %2;\n\t}"
+        : "+d"(a), "+d"(b)
+        : "d"(x), "r"(second));
+}
+__device__ __forceinline__ void add_if(float &a, float x, bool on)
+{
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p add.rn.f32 %0, %0, %1;\n\t}" : "+f"(a) : "f"(x), "r"((uint32_t)on));
+}
+__device__ __forceinline__ void add_if(double &a, double x, bool on)
+{
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p add.rn.f64 %0, %0, %1;\n\t}" : "+d"(a) : "d"(x), "r"((uint32_t)on));
+}
+
+template <int R> constexpr int wide_ids() { return R <= 8 ? 8 : 16; }
+// bits of a slot's member number
+template <int M> constexpr int member_bits() { return M == 1 ? 0 : M == 2 ? 1 : M <= 4 ? 2 : 3; }
+
+template <typename T, int R, int M> __device__ __forceinline__ void add_slots(T (&acc)[M][R], const T (&x)[R], uint32_t sel)
+{
+    if constexpr (M == 1) {
+        add_all<R>(acc[0], x);
+    } else {
+        constexpr int B = member_bits<M>();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if constexpr (M == 2) {
+                add_one_of(acc[0][r], acc[1][r], x[r], sel & (1u << r));
+            } else {
+                const uint32_t mine = sel & ((1u << B) - 1u) << (r * B);
+#pragma unroll
+                for (int m = 0; m < M; ++m) add_if(acc[m][r], x[r], mine == (uint32_t)m << (r * B));
+            }
+        }
+    }
+}
+
+template <typename T, int R, int M, int BR, int NBAT, int NP>
+__global__ void __launch_bounds__(kGatherThreads) k_gather_wide(GatherArgs a)
+{
+    constexpr int N = wide_ids<R>(), NC = N / 8, BPG = 32 / BR;   // BPG: batches in 32 entries
+    constexpr int PE = 16 / (int)sizeof(T);
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    // [color][lane]: bit p, piece lane + 32 p of the row is read; the members that the lane's slots take
+    __shared__ uint32_t need[16 * 32], member[16 * 32];
+    // [k][N / 8][32][8] byte offsets in a row slot; color 0: the zero behind the row
+    uint16_t *tab = reinterpret_cast<uint16_t *>(smem_raw);
+    unsigned char *ring_raw = smem_raw + (size_t)a.k * 32 * N * 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t row_bytes = ((uint32_t)a.nR * (uint32_t)sizeof(T) + 15u) / 16u * 16u, rs = row_bytes + 16u;
+    const int slot0 = blockIdx.y * (32 * R);
+    for (int i = threadIdx.x; i < 16 * 32; i += kGatherThreads) need[i] = member[i] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < a.k * 32 * N; i += kGatherThreads) {
+        const int d = i / (32 * N), c = i / 256 % NC, l = i / 8 % 32, r = c * 8 + i % 8;
+        const int slot = slot0 + r * 32 + l;
+        uint16_t x = 0xffffu;
+        if (d > 0 && r < R)
+            for (int m = 0; m < M; ++m) {
+                if (slot >= a.start[m + 1] - a.start[m]) break;
+                const uint16_t y = __ldg(a.idx + (size_t)(d - 1) * a.nA + a.start[m] + slot);
+                if (y == 0xffffu) continue;
+                x = y;
+                if (M > 1) atomicOr(&member[d * 32 + l], (uint32_t)m << (r * member_bits<M>()));
+            }
+        if (x != 0xffffu) atomicOr(&need[d * 32 + (x / PE & 31)], 1u << (x / PE >> 5));
+        tab[i] = (uint16_t)(x == 0xffffu ? row_bytes : (uint32_t)x * (uint32_t)sizeof(T));
+    }
+    if (blockIdx.y == 0) hub_part<T, 32>(a, ring_raw);
+    __syncthreads();
+    for (int i = threadIdx.x; i < kWarps * NBAT * BR; i += kGatherThreads)
+        *reinterpret_cast<uint4 *>(ring_raw + (size_t)i * rs + row_bytes) = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(ring_raw) + (uint32_t)(warp * NBAT * BR) * rs;
+    const uint32_t bs = BR * rs;   // bytes of a batch
+    const char *aux = reinterpret_cast<const char *>(a.aux) + lane * 16;
+    const uint32_t pitch_bytes = (uint32_t)a.pitch * (uint32_t)sizeof(T);
+    const uint16_t *mytab = tab + lane * 8;
+    const uint32_t *myneed = need + lane, *mymember = member + lane;
+    for (;;) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(a.ticket + blockIdx.y, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        int v0, v1;
+        if (!chunk_of(a.map, t, v0, v1)) break;
+        const int e0 = __ldg(a.off + v0), ends = __ldg(a.off + min(v0 + 1 + lane, v1));   // a chunk has at most 32 vertices
+        const int e1 = __shfl_sync(0xffffffffu, ends, v1 - v0 - 1);
+        const int nb = (e1 - e0 + BR - 1) / BR;
+        auto word = [&](int g) { const int e = e0 + g * 32 + lane; return e < e1 ? (uint32_t)__ldg(a.adjd + e) : 0u; };
+        // the words of the group of batch j (wA), of the next (wB) and of the one after
+        uint32_t wA = word(0), wB = word(1), wC = word(2);
+        auto issue = [&](int j, uint32_t w, uint32_t slot) {
+            if (j < nb) {
+#pragma unroll
+                for (int i = 0; i < BR; ++i) {
+                    const uint32_t x = __shfl_sync(0xffffffffu, w, j % BPG * BR + i);
+                    const uint32_t pm = myneed[(x >> 28) * 32];
+                    const char *src = aux + (uint64_t)(x & 0x0fffffffu) * pitch_bytes;
+                    const uint32_t dst = slot + (uint32_t)i * rs + (uint32_t)lane * 16u;
+#pragma unroll
+                    for (int p = 0; p < NP; ++p)
+                        if (pm >> p & 1u) cp_async16_s(dst + p * 512, src + p * 512);
+                }
+            }
+            cp_async_commit();
+        };
+        T acc[M][R];
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[m][r] = T(0);
+        __syncwarp();
+        uint32_t is = ring;
+#pragma unroll
+        for (int j = 0; j < NBAT - 1; ++j) {
+            issue(j, wA, is);
+            is += bs;
+        }
+        uint32_t cs = ring;
+        int v = v0, vend = __shfl_sync(0xffffffffu, ends, 0);
+        for (int j = 0; j < nb; ++j) {
+            issue(j + NBAT - 1, (j + NBAT - 1) / BPG == j / BPG ? wA : wB, is);
+            is = is == ring + (NBAT - 1) * bs ? ring : is + bs;
+            cp_async_wait<NBAT - 1>();
+            __syncwarp();
+            uint4 id[BR][NC];
+            uint32_t sel[BR];
+#pragma unroll
+            for (int i = 0; i < BR; ++i) {
+                const uint32_t d = __shfl_sync(0xffffffffu, wA, j % BPG * BR + i) >> 28;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) id[i][c] = *reinterpret_cast<const uint4 *>(mytab + (d * NC + c) * 256);
+                sel[i] = M > 1 ? mymember[d * 32] : 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < BR; ++i) {
+                const uint32_t row = cs + (uint32_t)i * rs;
+                T x[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const uint4 q = id[i][r / 8];
+                    const uint32_t w = (r & 7) < 2 ? q.x : (r & 7) < 4 ? q.y : (r & 7) < 6 ? q.z : q.w;
+                    x[r] = lds_elem(r & 1 ? add_hi(row, w) : add_lo(row, w), T(0));
+                }
+                add_slots<T, R, M>(acc, x, sel[i]);
+                if (e0 + j * BR + i + 1 == vend) {
+                    T *o = reinterpret_cast<T *>(a.out) + (size_t)v * a.out_pitch + slot0 + lane;
+#pragma unroll
+                    for (int m = 0; m < M; ++m) {
+                        const int n = a.start[m + 1] - a.start[m] - slot0 - lane;
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            if (r * 32 < n) o[a.start[m] + r * 32] = acc[m][r];
+                            acc[m][r] = T(0);
+                        }
+                    }
+                    ++v;
+                    vend = __shfl_sync(0xffffffffu, ends, (v - v0) & 31);
+                }
+            }
+            cs = cs == ring + (NBAT - 1) * bs ? ring : cs + bs;
+            __syncwarp();
+            if (j % BPG == BPG - 1) {
+                wA = wB;
+                wB = wC;
+                wC = word(j / BPG + 3);
+            }
+        }
+        cp_async_wait<0>();
+    }
+}
+
+// Narrow.  U neighbours in flight a lane; a slot of which no set holds the
+// neighbour's color loads nothing.  A table entry: the row's column (13 bits)
+// and the slot's member.
+template <int R> struct Ids { static constexpr int n = R <= 1 ? 1 : R <= 2 ? 2 : R <= 4 ? 4 : R <= 8 ? 8 : 16; };
+
+template <int N> __device__ __forceinline__ void load_ids(const uint16_t *p, uint32_t (&w)[(N + 1) / 2])
+{
+    if constexpr (N == 1) {
+        w[0] = *p;
+    } else if constexpr (N == 2) {
+        w[0] = *reinterpret_cast<const uint32_t *>(p);
+    } else if constexpr (N == 4) {
+        const uint2 t = *reinterpret_cast<const uint2 *>(p);
+        w[0] = t.x; w[1] = t.y;
+    } else {
+#pragma unroll
+        for (int i = 0; i < N / 8; ++i) {
+            const uint4 t = *(reinterpret_cast<const uint4 *>(p) + i);
+            w[4 * i] = t.x; w[4 * i + 1] = t.y; w[4 * i + 2] = t.z; w[4 * i + 3] = t.w;
+        }
+    }
+}
+
+__device__ __forceinline__ float ld_if(const float *p, bool on)
+{
+    float x;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+        : "=f"(x)
+        : "l"(p), "r"((uint32_t)on));
+    return x;
+}
+__device__ __forceinline__ double ld_if(const double *p, bool on)
+{
+    double x;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t@q ld.global.nc.f64 %0, [%1];\n\t}"
+        : "=d"(x)
+        : "l"(p), "r"((uint32_t)on));
+    return x;
+}
+
+template <typename T, int G, int R, int M, int U, int GH> __global__ void __launch_bounds__(kGatherThreads) k_gather(GatherArgs a)
+{
+    constexpr int N = Ids<R>::n;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint16_t *tab = reinterpret_cast<uint16_t *>(smem_raw);   // [k][G][N]; color 0: adds nothing
+    const int slot0 = blockIdx.y * (G * R);
+    for (int i = threadIdx.x; i < a.k * G * N; i += kGatherThreads) {
+        const int d = i / (G * N), l = (i - d * (G * N)) / N, r = i % N;
+        const int slot = slot0 + r * G + l;
+        uint16_t x = 0xffffu;
+        if (d > 0 && r < R)
+            for (int m = 0; m < M; ++m) {
+                if (slot >= a.start[m + 1] - a.start[m]) break;
+                const uint16_t y = __ldg(a.idx + (size_t)(d - 1) * a.nA + a.start[m] + slot);
+                if (y != 0xffffu) x = (uint16_t)(y | m << 13);
+            }
+        tab[i] = x;
+    }
+    unsigned char *rest = smem_raw + ((size_t)a.k * G * N * 2 + 15) / 16 * 16;
+    if (blockIdx.y == 0) hub_part<T, GH>(a, rest);
+    __syncthreads();
+    T *sacc = reinterpret_cast<T *>(rest) + threadIdx.x;   // M > 2: [R][M][threads], a thread's own
+    const int lane = threadIdx.x & 31, lg = lane % G, grp = lane / G;
+    const uint16_t *mytab = tab + lg * N;
+    const T *aux = reinterpret_cast<const T *>(a.aux);
+    for (;;) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(a.ticket + blockIdx.y, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        int v0, v1;
+        if (!chunk_of(a.map, t, v0, v1)) break;
+        for (int v = v0 + grp; v < v1; v += 32 / G) {
+            T acc[M][R];
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    acc[m][r] = T(0);
+                    if (M > 2) sacc[(r * M + m) * kGatherThreads] = T(0);
+                }
+            const int beg = __ldg(a.off + v), end = __ldg(a.off + v + 1);
+            uint32_t w[U];   // the next batch's neighbour words, a batch ahead
+#pragma unroll
+            for (int u = 0; u < U; ++u) w[u] = beg + u < end ? (uint32_t)__ldg(a.adjd + beg + u) : 0u;
+            for (int e = beg; e < end; e += U) {
+                T x[U][R];
+                uint32_t mem[U][R];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    uint32_t id[(N + 1) / 2];
+                    load_ids<N>(mytab + (w[u] >> 28) * (G * N), id);
+                    const T *row = aux + (size_t)(w[u] & 0x0fffffffu) * a.pitch;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const uint32_t c = r & 1 ? id[r / 2] >> 16 : id[r / 2] & 0xffffu;
+                        x[u][r] = ld_if(row + (c & 0x1fffu), c != 0xffffu);
+                        // the member; where there is none, x is 0 and any will do
+                        mem[u][r] = M > 2 ? (c == 0xffffu ? 0u : c >> 13) : c & 0x2000u;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) w[u] = e + U + u < end ? (uint32_t)__ldg(a.adjd + e + U + u) : 0u;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        if constexpr (M == 1) {
+                            acc[0][r] = add_rn(acc[0][r], x[u][r]);
+                        } else if constexpr (M == 2) {
+                            add_one_of(acc[0][r], acc[1][r], x[u][r], mem[u][r]);
+                        } else {
+                            T *p = sacc + (r * M + mem[u][r]) * kGatherThreads;
+                            *p = add_rn(*p, x[u][r]);
+                        }
+                    }
+            }
+            T *o = reinterpret_cast<T *>(a.out) + (size_t)v * a.out_pitch + slot0;
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if (slot0 + r * G + lg < a.start[m + 1] - a.start[m])
+                        o[a.start[m] + r * G + lg] = M > 2 ? sacc[(r * M + m) * kGatherThreads] : acc[m][r];
+        }
+    }
+}
+
+namespace {
+
+// CTAs of a kernel an SM holds; the answer for the last (device, size) is kept
+// a kernel (the driver's takes microseconds).
+template <typename F> int resident(F kern, size_t smem, std::atomic<uint64_t> &last)
+{
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t key = (uint64_t)dev << 40 | (uint64_t)smem << 8, got = last.load(std::memory_order_relaxed);
+    if ((got & ~(uint64_t)0xff) == key && (got & 0xff)) return (int)(got & 0xff);
+    // static shared memory counts against the default limit too
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kGatherThreads, smem) != cudaSuccess || n < 1) n = 1;
+    last.store(key | (uint64_t)std::min(n, 255), std::memory_order_relaxed);
+    return n;
+}
+
+int gather_grid(const GatherArgs &a, int per_sm, int sm_count, int hub_cols)
+{
+    const int64_t items = (int64_t)a.hubs * ((a.nA + hub_cols - 1) / hub_cols);
+    const int64_t want = (a.map.base[a.map.n] + kWarps - 1) / kWarps + items;
+    return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count * per_sm, want));
+}
+
+template <typename T, int G, int R, int M, int U, int GH> void go_narrow_h(const GatherArgs &a, int sm_count, cudaStream_t st)
+{
+    const size_t sacc = M > 2 ? (size_t)R * M * kGatherThreads * sizeof(T) : 0;
+    const size_t smem = ((size_t)a.k * G * Ids<R>::n * 2 + 15) / 16 * 16 + std::max(sacc, a.hubs > 0 ? hub_bytes<T, GH>() : 0);
+    auto kern = k_gather<T, G, R, M, U, GH>;
+    static std::atomic<uint64_t> last{0};
+    const int per_sm = resident(kern, smem, last);
+    kern<<<dim3(gather_grid(a, per_sm, sm_count, GH), (a.slots + G * R - 1) / (G * R)), kGatherThreads, smem, st>>>(a);
+}
+
+template <typename T, int G, int R, int M, int U> void go_narrow(const GatherArgs &a, int sm_count, cudaStream_t st)
+{
+    if constexpr (G * R * M == 1) return go_narrow_h<T, G, R, M, U, 1>(a, sm_count, st);
+    if constexpr (G * R * M <= 8) return go_narrow_h<T, G, R, M, U, 8>(a, sm_count, st);
+    if (a.nA <= 8) return go_narrow_h<T, G, R, M, U, 8>(a, sm_count, st);
+    if (a.nA <= 16) return go_narrow_h<T, G, R, M, U, 16>(a, sm_count, st);
+    return go_narrow_h<T, G, R, M, U, 32>(a, sm_count, st);
+}
+
+template <typename T, int M> void pick_narrow(const GatherArgs &a, int sm_count, cudaStream_t st)
+{
+    const int n = a.slots;
+    if constexpr (M == 1)
+        if (n <= 1) return go_narrow<T, 1, 1, 1, 8>(a, sm_count, st);
+    if constexpr (M <= 2)
+        if (n <= 4) return go_narrow<T, 4, 1, M, 8>(a, sm_count, st);
+    if constexpr (M <= 4)
+        if (n <= 8) return go_narrow<T, 8, 1, M, 8>(a, sm_count, st);
+    if (n <= 16) return go_narrow<T, 16, 1, M, 8>(a, sm_count, st);
+    if (n <= 32) return go_narrow<T, 32, 1, M, 8>(a, sm_count, st);
+    if (n <= 64) return go_narrow<T, 32, 2, M, 4>(a, sm_count, st);
+    return go_narrow<T, 32, 4, M, 2>(a, sm_count, st);
+}
+
+// The ring: batches of two rows, four of them (three of the longest rows), so
+// that two CTAs of eight warps fit an SM; of four rows where they are short.
+constexpr size_t kWideSmem = 108 * 1024;
+inline int wide_ring(size_t row_bytes) { return row_bytes <= 512 ? 16 : row_bytes <= 1536 ? 8 : 6; }
+template <typename T> size_t wide_smem(const GatherArgs &a, int ids)
+{
+    const size_t rb = ((size_t)a.nR * sizeof(T) + 15) / 16 * 16;
+    return (size_t)a.k * 32 * ids * 2 +
+           std::max((size_t)kWarps * wide_ring(rb) * (rb + 16), a.hubs > 0 ? hub_bytes<T, 32>() : 0);
+}
+
+template <typename T, int R, int M, int BR, int NBAT, int NP> void go_wide_n(const GatherArgs &a, int sm_count, cudaStream_t st)
+{
+    const size_t smem = wide_smem<T>(a, wide_ids<R>());
+    auto kern = k_gather_wide<T, R, M, BR, NBAT, NP>;
+    static std::atomic<uint64_t> last{0};
+    const int per_sm = resident(kern, smem, last);
+    kern<<<dim3(gather_grid(a, per_sm, sm_count, 32), (a.slots + 32 * R - 1) / (32 * R)), kGatherThreads, smem, st>>>(a);
+}
+
+// NP: 16-byte pieces of a row a lane
+template <typename T, int R, int M> void go_wide(const GatherArgs &a, int sm_count, cudaStream_t st)
+{
+    const size_t rb = ((size_t)a.nR * sizeof(T) + 15) / 16 * 16;
+    switch (wide_ring(rb)) {
+    case 16: return go_wide_n<T, R, M, 4, 4, 1>(a, sm_count, st);
+    case 8: return go_wide_n<T, R, M, 2, 4, 3>(a, sm_count, st);
+    default: return rb <= 2048 ? go_wide_n<T, R, M, 2, 3, 4>(a, sm_count, st) : go_wide_n<T, R, M, 2, 3, 8>(a, sm_count, st);
+    }
+}
+
+template <typename T> bool is_wide(const GatherArgs &a)
+{
+    return a.slots > 32 && a.nR >= 32 && a.nR * sizeof(T) <= 4096 && wide_smem<T>(a, a.slots <= 256 ? 8 : 16) <= kWideSmem;
+}
+
+template <typename T, int M> void pick_wide(const GatherArgs &a, int sm_count, cudaStream_t st)
+{
+    const int n = a.slots;
+    if (n <= 64) return go_wide<T, 2, M>(a, sm_count, st);
+    if (n <= 96) return go_wide<T, 3, M>(a, sm_count, st);
+    if (n <= 128) return go_wide<T, 4, M>(a, sm_count, st);
+    if (n <= 192) return go_wide<T, 6, M>(a, sm_count, st);
+    if constexpr (M <= 2) {
+        if (n > 256 && n <= 352) return go_wide<T, 11, M>(a, sm_count, st);
+        if (n > 256 && n <= 480) return go_wide<T, 15, M>(a, sm_count, st);
+    }
+    return go_wide<T, 8, M>(a, sm_count, st);
+}
+
+template <typename T, int M> void pick_gather(const GatherArgs &a, int sm_count, cudaStream_t st)
+{
+    if (is_wide<T>(a)) pick_wide<T, M>(a, sm_count, st);
+    else pick_narrow<T, M>(a, sm_count, st);
+}
+
+template <typename T> void launch_gather_t(const GatherArgs &a, int sm_count, cudaStream_t st)
+{
+    switch (a.members) {
+    case 1: return pick_gather<T, 1>(a, sm_count, st);
+    case 2: return pick_gather<T, 2>(a, sm_count, st);
+    case 3: return pick_gather<T, 3>(a, sm_count, st);
+    case 4: return pick_gather<T, 4>(a, sm_count, st);
+    default: return pick_gather<T, 5>(a, sm_count, st);
+    }
+}
+
+}  // namespace
+
+}  // namespace rt
+}  // namespace sg

@@ -1,0 +1,9 @@
+#include "rooted_gather.cuh"
+
+namespace sg {
+namespace rt {
+
+void launch_gather_f64(const GatherArgs &a, int sm_count, cudaStream_t st) { launch_gather_t<double>(a, sm_count, st); }
+
+}  // namespace rt
+}  // namespace sg

@@ -135,13 +135,20 @@ __device__ __forceinline__ double block_sum_partials(const double *p, int n, dou
                                                      double *pp)
 {
     double s = 0.0, c = 0.0, plain = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double x = p[i];
-        plain = __dadd_rn(plain, x);
-        const double y = __dadd_rn(x, -c);
-        const double t = __dadd_rn(s, y);
-        c = __dadd_rn(__dadd_rn(t, -s), -y);
-        s = t;
+    // eight partials a thread in flight: the adds are a chain, the loads need not wait for it
+    for (int i0 = threadIdx.x; i0 < n; i0 += 8 * blockDim.x) {
+        double x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = i0 + u * (int)blockDim.x < n ? __ldg(p + i0 + u * blockDim.x) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (i0 + u * (int)blockDim.x >= n) break;
+            plain = __dadd_rn(plain, x[u]);
+            const double y = __dadd_rn(x[u], -c);
+            const double t = __dadd_rn(s, y);
+            c = __dadd_rn(__dadd_rn(t, -s), -y);
+            s = t;
+        }
     }
     ss[threadIdx.x] = s;
     cc[threadIdx.x] = c;
