@@ -151,10 +151,13 @@ template <typename T, int GH> __device__ __forceinline__ void hub_part(const Gat
 }
 
 // Wide.  A warp walks the neighbour entries of its vertices as one stream
-// through a ring of NBAT batches of BR rows in shared memory (cp.async, the
-// 16-byte pieces that the neighbour's color needs).  A lane then reads, for
-// each of its columns, the element the color points at (a zero behind the row
-// where it points at none).
+// through a ring of RR rows in shared memory, BR of them a copy group
+// (cp.async, the 16-byte pieces that the neighbour's color needs).  A lane
+// then reads, for each of its slots, the element the color points at (a zero
+// behind the row where it points at none).  What depends on the color and
+// the lane alone (which pieces, which of a slot's sets) is a bit per color in
+// registers, tested against 1 << color; the offsets are a table in shared
+// memory, eight to a load.
 __device__ __forceinline__ float lds_elem(uint32_t addr, float)
 {
     float x;
@@ -202,53 +205,37 @@ __device__ __forceinline__ void add_one_of(double &a, double &b, double x, uint3
         : "+d"(a), "+d"(b)
         : "d"(x), "r"(second));
 }
-__device__ __forceinline__ void add_if(float &a, float x, bool on)
+__device__ __forceinline__ void add_if(float &a, float x, uint32_t on)
 {
-    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p add.rn.f32 %0, %0, %1;\n\t}" : "+f"(a) : "f"(x), "r"((uint32_t)on));
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p add.rn.f32 %0, %0, %1;\n\t}" : "+f"(a) : "f"(x), "r"(on));
 }
-__device__ __forceinline__ void add_if(double &a, double x, bool on)
+__device__ __forceinline__ void add_if(double &a, double x, uint32_t on)
 {
-    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p add.rn.f64 %0, %0, %1;\n\t}" : "+d"(a) : "d"(x), "r"((uint32_t)on));
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p add.rn.f64 %0, %0, %1;\n\t}" : "+d"(a) : "d"(x), "r"(on));
 }
+
+// bytes between the ring's rows: the row and a zero, in whole lines as the table's rows
+__host__ __device__ inline uint32_t wide_stride(uint32_t row_bytes) { return (row_bytes + 16u + 127u) / 128u * 128u; }
 
 template <int R> constexpr int wide_ids() { return R <= 8 ? 8 : 16; }
-// bits of a slot's member number
-template <int M> constexpr int member_bits() { return M == 1 ? 0 : M == 2 ? 1 : M <= 4 ? 2 : 3; }
 
-template <typename T, int R, int M> __device__ __forceinline__ void add_slots(T (&acc)[M][R], const T (&x)[R], uint32_t sel)
-{
-    if constexpr (M == 1) {
-        add_all<R>(acc[0], x);
-    } else {
-        constexpr int B = member_bits<M>();
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            if constexpr (M == 2) {
-                add_one_of(acc[0][r], acc[1][r], x[r], sel & (1u << r));
-            } else {
-                const uint32_t mine = sel & ((1u << B) - 1u) << (r * B);
-#pragma unroll
-                for (int m = 0; m < M; ++m) add_if(acc[m][r], x[r], mine == (uint32_t)m << (r * B));
-            }
-        }
-    }
-}
-
-template <typename T, int R, int M, int BR, int NBAT, int NP>
+template <typename T, int R, int M, int RR, int BR, int NP>
 __global__ void __launch_bounds__(kGatherThreads) k_gather_wide(GatherArgs a)
 {
-    constexpr int N = wide_ids<R>(), NC = N / 8, BPG = 32 / BR;   // BPG: batches in 32 entries
+    constexpr int N = wide_ids<R>(), NC = N / 8, PF = RR - BR;   // PF: rows copied ahead
     constexpr int PE = 16 / (int)sizeof(T);
+    constexpr int MB = M == 1 ? 0 : M == 2 ? 1 : M;              // member masks a slot (two members: the second's)
+    static_assert(32 % RR == 0 && RR % BR == 0 && PF % BR == 0 && PF > 0, "a ring divides 32 entries");
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    // [color][lane]: bit p, piece lane + 32 p of the row is read; the members that the lane's slots take
-    __shared__ uint32_t need[16 * 32], member[16 * 32];
+    __shared__ uint32_t need[NP][32], member[MB ? MB * R : 1][32];   // [..][lane]: a bit per color
     // [k][N / 8][32][8] byte offsets in a row slot; color 0: the zero behind the row
     uint16_t *tab = reinterpret_cast<uint16_t *>(smem_raw);
-    unsigned char *ring_raw = smem_raw + (size_t)a.k * 32 * N * 2;
+    unsigned char *ring_raw = smem_raw + (size_t)a.k * 32 * N * 2;   // a multiple of 512 bytes
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t row_bytes = ((uint32_t)a.nR * (uint32_t)sizeof(T) + 15u) / 16u * 16u, rs = row_bytes + 16u;
+    const uint32_t row_bytes = ((uint32_t)a.nR * (uint32_t)sizeof(T) + 15u) / 16u * 16u, rs = wide_stride(row_bytes);
     const int slot0 = blockIdx.y * (32 * R);
-    for (int i = threadIdx.x; i < 16 * 32; i += kGatherThreads) need[i] = member[i] = 0;
+    for (int i = threadIdx.x; i < NP * 32; i += kGatherThreads) (&need[0][0])[i] = 0;
+    for (int i = threadIdx.x; i < MB * R * 32; i += kGatherThreads) (&member[0][0])[i] = 0;
     __syncthreads();
     for (int i = threadIdx.x; i < a.k * 32 * N; i += kGatherThreads) {
         const int d = i / (32 * N), c = i / 256 % NC, l = i / 8 % 32, r = c * 8 + i % 8;
@@ -260,48 +247,51 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_wide(GatherArgs a)
                 const uint16_t y = __ldg(a.idx + (size_t)(d - 1) * a.nA + a.start[m] + slot);
                 if (y == 0xffffu) continue;
                 x = y;
-                if (M > 1) atomicOr(&member[d * 32 + l], (uint32_t)m << (r * member_bits<M>()));
+                if (MB == 1 && m == 1) atomicOr(&member[r][l], 1u << d);
+                if (MB > 1) atomicOr(&member[r * MB + m][l], 1u << d);
             }
-        if (x != 0xffffu) atomicOr(&need[d * 32 + (x / PE & 31)], 1u << (x / PE >> 5));
+        if (x != 0xffffu) {   // whole sectors: the two pieces of 32 bytes
+            const int q = x / PE & ~1;
+            atomicOr(&need[q >> 5][q & 31], 1u << d);
+            if ((uint32_t)(q + 1) * 16 < row_bytes) atomicOr(&need[q >> 5][(q & 31) + 1], 1u << d);
+        }
         tab[i] = (uint16_t)(x == 0xffffu ? row_bytes : (uint32_t)x * (uint32_t)sizeof(T));
     }
     if (blockIdx.y == 0) hub_part<T, 32>(a, ring_raw);
     __syncthreads();
-    for (int i = threadIdx.x; i < kWarps * NBAT * BR; i += kGatherThreads)
+    for (int i = threadIdx.x; i < kWarps * RR; i += kGatherThreads)
         *reinterpret_cast<uint4 *>(ring_raw + (size_t)i * rs + row_bytes) = make_uint4(0, 0, 0, 0);
+    uint32_t nd[NP], mb[MB ? MB * R : 1];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) nd[p] = need[p][lane];
+#pragma unroll
+    for (int i = 0; i < MB * R; ++i) mb[i] = member[i][lane];
     __syncthreads();
-    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(ring_raw) + (uint32_t)(warp * NBAT * BR) * rs;
-    const uint32_t bs = BR * rs;   // bytes of a batch
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(ring_raw) + (uint32_t)(warp * RR) * rs;
     const char *aux = reinterpret_cast<const char *>(a.aux) + lane * 16;
     const uint32_t pitch_bytes = (uint32_t)a.pitch * (uint32_t)sizeof(T);
     const uint16_t *mytab = tab + lane * 8;
-    const uint32_t *myneed = need + lane, *mymember = member + lane;
     for (;;) {
         int t = 0;
         if (lane == 0) t = atomicAdd(a.ticket + blockIdx.y, 1);
         t = __shfl_sync(0xffffffffu, t, 0);
         int v0, v1;
         if (!chunk_of(a.map, t, v0, v1)) break;
-        const int e0 = __ldg(a.off + v0), ends = __ldg(a.off + min(v0 + 1 + lane, v1));   // a chunk has at most 32 vertices
-        const int e1 = __shfl_sync(0xffffffffu, ends, v1 - v0 - 1);
-        const int nb = (e1 - e0 + BR - 1) / BR;
-        auto word = [&](int g) { const int e = e0 + g * 32 + lane; return e < e1 ? (uint32_t)__ldg(a.adjd + e) : 0u; };
-        // the words of the group of batch j (wA), of the next (wB) and of the one after
+        const int e0 = __ldg(a.off + v0), ends = __ldg(a.off + min(v0 + 1 + lane, v1)) - e0;   // a chunk has at most 32 vertices
+        const int n = __shfl_sync(0xffffffffu, ends, v1 - v0 - 1);
+        auto word = [&](int g) { return g * 32 + lane < n ? (uint32_t)__ldg(a.adjd + e0 + g * 32 + lane) : 0u; };
+        // the words of 32 entries (wA), of the next 32 (wB) and of those after
         uint32_t wA = word(0), wB = word(1), wC = word(2);
-        auto issue = [&](int j, uint32_t w, uint32_t slot) {
-            if (j < nb) {
+        uint32_t color[RR];   // of the ring's rows
+        auto issue = [&](int rr, uint32_t w, int from) {
+            const uint32_t x = __shfl_sync(0xffffffffu, w, from);
+            color[rr] = x >> 28;
+            const uint32_t bit = 1u << (x >> 28);
+            const char *src = aux + (uint64_t)(x & 0x0fffffffu) * pitch_bytes;
+            const uint32_t dst = ring + (uint32_t)rr * rs + (uint32_t)lane * 16u;
 #pragma unroll
-                for (int i = 0; i < BR; ++i) {
-                    const uint32_t x = __shfl_sync(0xffffffffu, w, j % BPG * BR + i);
-                    const uint32_t pm = myneed[(x >> 28) * 32];
-                    const char *src = aux + (uint64_t)(x & 0x0fffffffu) * pitch_bytes;
-                    const uint32_t dst = slot + (uint32_t)i * rs + (uint32_t)lane * 16u;
-#pragma unroll
-                    for (int p = 0; p < NP; ++p)
-                        if (pm >> p & 1u) cp_async16_s(dst + p * 512, src + p * 512);
-                }
-            }
-            cp_async_commit();
+            for (int p = 0; p < NP; ++p)
+                if (nd[p] & bit) cp_async16_s(dst + p * 512, src + p * 512);
         };
         T acc[M][R];
 #pragma unroll
@@ -309,60 +299,76 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_wide(GatherArgs a)
 #pragma unroll
             for (int r = 0; r < R; ++r) acc[m][r] = T(0);
         __syncwarp();
-        uint32_t is = ring;
 #pragma unroll
-        for (int j = 0; j < NBAT - 1; ++j) {
-            issue(j, wA, is);
-            is += bs;
+        for (int q = 0; q < PF; ++q) {
+            issue(q, wA, q);
+            if (q % BR == BR - 1) cp_async_commit();
         }
-        uint32_t cs = ring;
         int v = v0, vend = __shfl_sync(0xffffffffu, ends, 0);
-        for (int j = 0; j < nb; ++j) {
-            issue(j + NBAT - 1, (j + NBAT - 1) / BPG == j / BPG ? wA : wB, is);
-            is = is == ring + (NBAT - 1) * bs ? ring : is + bs;
-            cp_async_wait<NBAT - 1>();
-            __syncwarp();
-            uint4 id[BR][NC];
-            uint32_t sel[BR];
+        for (int b = 0; b < n; b += RR) {
+            const int at = b & 31;                       // in wA
+            const uint32_t wN = at + RR == 32 ? wB : wA; // of the entries RR further
 #pragma unroll
-            for (int i = 0; i < BR; ++i) {
-                const uint32_t d = __shfl_sync(0xffffffffu, wA, j % BPG * BR + i) >> 28;
+            for (int q = 0; q < RR; q += BR) {
+                if (b + q >= n) break;
 #pragma unroll
-                for (int c = 0; c < NC; ++c) id[i][c] = *reinterpret_cast<const uint4 *>(mytab + (d * NC + c) * 256);
-                sel[i] = M > 1 ? mymember[d * 32] : 0u;
-            }
-#pragma unroll
-            for (int i = 0; i < BR; ++i) {
-                const uint32_t row = cs + (uint32_t)i * rs;
-                T x[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const uint4 q = id[i][r / 8];
-                    const uint32_t w = (r & 7) < 2 ? q.x : (r & 7) < 4 ? q.y : (r & 7) < 6 ? q.z : q.w;
-                    x[r] = lds_elem(r & 1 ? add_hi(row, w) : add_lo(row, w), T(0));
+                for (int i = 0; i < BR; ++i) {
+                    const int f = q + PF + i;
+                    issue(f % RR, f < RR ? wA : wN, (at + f) & 31);
                 }
-                add_slots<T, R, M>(acc, x, sel[i]);
-                if (e0 + j * BR + i + 1 == vend) {
-                    T *o = reinterpret_cast<T *>(a.out) + (size_t)v * a.out_pitch + slot0 + lane;
+                cp_async_commit();
+                cp_async_wait<PF / BR>();
+                __syncwarp();
+                uint4 id[BR][NC];
 #pragma unroll
-                    for (int m = 0; m < M; ++m) {
-                        const int n = a.start[m + 1] - a.start[m] - slot0 - lane;
+                for (int i = 0; i < BR; ++i)
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        id[i][c] = *reinterpret_cast<const uint4 *>(mytab + (color[q + i] * NC + c) * 256);
+#pragma unroll
+                for (int i = 0; i < BR; ++i) {
+                    const uint32_t row = ring + (uint32_t)(q + i) * rs, bit = 1u << color[q + i];
+                    T x[R];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const uint4 z = id[i][r / 8];
+                        const uint32_t w = (r & 7) < 2 ? z.x : (r & 7) < 4 ? z.y : (r & 7) < 6 ? z.z : z.w;
+                        x[r] = lds_elem(r & 1 ? add_hi(row, w) : add_lo(row, w), T(0));
+                    }
+                    if constexpr (M == 1) {
+                        add_all<R>(acc[0], x);
+                    } else {
 #pragma unroll
                         for (int r = 0; r < R; ++r) {
-                            if (r * 32 < n) o[a.start[m] + r * 32] = acc[m][r];
-                            acc[m][r] = T(0);
+                            if constexpr (M == 2) {
+                                add_one_of(acc[0][r], acc[1][r], x[r], mb[r] & bit);
+                            } else {
+#pragma unroll
+                                for (int m = 0; m < M; ++m) add_if(acc[m][r], x[r], mb[r * MB + m] & bit);
+                            }
                         }
                     }
-                    ++v;
-                    vend = __shfl_sync(0xffffffffu, ends, (v - v0) & 31);
+                    if (b + q + i + 1 == vend) {
+                        T *o = reinterpret_cast<T *>(a.out) + (size_t)v * a.out_pitch + slot0 + lane;
+#pragma unroll
+                        for (int m = 0; m < M; ++m) {
+                            const int cols = a.start[m + 1] - a.start[m] - slot0 - lane;
+#pragma unroll
+                            for (int r = 0; r < R; ++r) {
+                                if (r * 32 < cols) o[a.start[m] + r * 32] = acc[m][r];
+                                acc[m][r] = T(0);
+                            }
+                        }
+                        ++v;
+                        vend = __shfl_sync(0xffffffffu, ends, (v - v0) & 31);
+                    }
                 }
+                __syncwarp();
             }
-            cs = cs == ring + (NBAT - 1) * bs ? ring : cs + bs;
-            __syncwarp();
-            if (j % BPG == BPG - 1) {
+            if (at + RR == 32) {
                 wA = wB;
                 wB = wC;
-                wC = word(j / BPG + 3);
+                wC = word((b >> 5) + 3);
             }
         }
         cp_async_wait<0>();
@@ -555,21 +561,23 @@ template <typename T, int M> void pick_narrow(const GatherArgs &a, int sm_count,
     return go_narrow<T, 32, 4, M, 2>(a, sm_count, st);
 }
 
-// The ring: batches of two rows, four of them (three of the longest rows), so
-// that two CTAs of eight warps fit an SM; of four rows where they are short.
-constexpr size_t kWideSmem = 108 * 1024;
-inline int wide_ring(size_t row_bytes) { return row_bytes <= 512 ? 16 : row_bytes <= 1536 ? 8 : 6; }
+// Rows in the ring.  Eight (sixteen short ones, four of the longest) measured
+// fastest: at 131,072 vertices of degree 32 and 12 colors, rows of 1848 bytes
+// take 0.82 ms with four and three CTAs an SM, 0.75 with eight and one; rows of
+// 1320 bytes 0.71 with sixteen and one CTA, 0.55 with eight and two.
+constexpr size_t kWideSmem = 215 * 1024;
+inline int wide_ring(size_t row_bytes) { return row_bytes <= 512 ? 16 : row_bytes <= 2816 ? 8 : 4; }
 template <typename T> size_t wide_smem(const GatherArgs &a, int ids)
 {
     const size_t rb = ((size_t)a.nR * sizeof(T) + 15) / 16 * 16;
     return (size_t)a.k * 32 * ids * 2 +
-           std::max((size_t)kWarps * wide_ring(rb) * (rb + 16), a.hubs > 0 ? hub_bytes<T, 32>() : 0);
+           std::max((size_t)kWarps * wide_ring(rb) * wide_stride((uint32_t)rb), a.hubs > 0 ? hub_bytes<T, 32>() : 0);
 }
 
-template <typename T, int R, int M, int BR, int NBAT, int NP> void go_wide_n(const GatherArgs &a, int sm_count, cudaStream_t st)
+template <typename T, int R, int M, int RR, int BR, int NP> void go_wide_n(const GatherArgs &a, int sm_count, cudaStream_t st)
 {
     const size_t smem = wide_smem<T>(a, wide_ids<R>());
-    auto kern = k_gather_wide<T, R, M, BR, NBAT, NP>;
+    auto kern = k_gather_wide<T, R, M, RR, BR, NP>;
     static std::atomic<uint64_t> last{0};
     const int per_sm = resident(kern, smem, last);
     kern<<<dim3(gather_grid(a, per_sm, sm_count, 32), (a.slots + 32 * R - 1) / (32 * R)), kGatherThreads, smem, st>>>(a);
@@ -580,9 +588,12 @@ template <typename T, int R, int M> void go_wide(const GatherArgs &a, int sm_cou
 {
     const size_t rb = ((size_t)a.nR * sizeof(T) + 15) / 16 * 16;
     switch (wide_ring(rb)) {
-    case 16: return go_wide_n<T, R, M, 4, 4, 1>(a, sm_count, st);
-    case 8: return go_wide_n<T, R, M, 2, 4, 3>(a, sm_count, st);
-    default: return rb <= 2048 ? go_wide_n<T, R, M, 2, 3, 4>(a, sm_count, st) : go_wide_n<T, R, M, 2, 3, 8>(a, sm_count, st);
+    case 16: return go_wide_n<T, R, M, 16, 4, 1>(a, sm_count, st);
+    case 8:
+        if (rb <= 1536) return go_wide_n<T, R, M, 8, 4, 3>(a, sm_count, st);
+        if (rb <= 2048) return go_wide_n<T, R, M, 8, 2, 4>(a, sm_count, st);
+        return go_wide_n<T, R, M, 8, 2, 8>(a, sm_count, st);
+    default: return go_wide_n<T, R, M, 4, 2, 8>(a, sm_count, st);
     }
 }
 
