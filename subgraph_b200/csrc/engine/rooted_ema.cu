@@ -21,6 +21,8 @@ template <typename T, bool FUSED> __global__ void __launch_bounds__(kEmaThreads)
     const int v0 = blockIdx.x * TV, tv = min(TV, a.V - v0);
     ema_rows(reinterpret_cast<const T *>(a.agg), a.agg_pitch, a.perm_a, a.nA, a.color, v0, tv, agg_s, RS);
     ema_rows(reinterpret_cast<const T *>(a.main), a.main_pitch, a.perm_m, a.nM, a.color, v0, tv, main_s, RS);
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (a.is_root) {
@@ -42,7 +44,7 @@ template <typename T, bool FUSED> __global__ void __launch_bounds__(kEmaThreads)
     // lane: four independent chains in split order
     const int vi = lane % TV, sub = lane / TV, per = 32 / TV;
     const int ng = (a.nO + 3) / 4;
-    for (int g = warp * per + sub; g < ng; g += kEmaThreads / 32 * per) {
+    for (int g = warp * per + sub; g < ng; g += (int)(blockDim.x >> 5) * per) {
         const uint4 *sp = reinterpret_cast<const uint4 *>(a.split) + g;
         const int step = a.split_stride / 4;
         T c0 = T(0), c1 = T(0), c2 = T(0), c3 = T(0);
@@ -102,7 +104,7 @@ void launch_ema(const EmaArgs &a0, bool fp64, cudaStream_t st)
     const int tiles = (a.V + a.tile_v - 1) / a.tile_v;
     auto go = [&](auto kern) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<tiles, kEmaThreads, smem, st>>>(a);
+        kern<<<tiles, a.is_root ? 128 : ema_threads(smem), smem, st>>>(a);
     };
     if (fp64) go(k_ema<double, false>);
     else if (a.fused) go(k_ema<float, true>);
