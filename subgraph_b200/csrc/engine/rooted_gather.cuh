@@ -375,9 +375,13 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_wide(GatherArgs a)
     }
 }
 
-// Narrow.  U neighbours in flight a lane; a slot of which no set holds the
-// neighbour's color loads nothing.  A table entry: the row's column (13 bits)
-// and the slot's member.
+// Narrow.  U neighbours in flight a lane, their words loaded once a group of
+// G lanes (a batch ahead) and passed round by shuffles.  A slot of which no set
+// holds the neighbour's color loads nothing: a bit per color and slot in a
+// register, as for which of two sets it is; with more sets a slot the member
+// is in the table's entry (above the column's 13 bits) and the sums are in
+// shared memory.  The warp's vertices (of like degree) take as many batches as
+// the longest list of them.
 template <int R> struct Ids { static constexpr int n = R <= 1 ? 1 : R <= 2 ? 2 : R <= 4 ? 4 : R <= 8 ? 8 : 16; };
 
 template <int N> __device__ __forceinline__ void load_ids(const uint16_t *p, uint32_t (&w)[(N + 1) / 2])
@@ -398,38 +402,44 @@ template <int N> __device__ __forceinline__ void load_ids(const uint16_t *p, uin
     }
 }
 
-__device__ __forceinline__ float ld_if(const float *p, bool on)
+__device__ __forceinline__ float ld_if(const float *p, uint32_t on)
 {
     float x;
     asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
         : "=f"(x)
-        : "l"(p), "r"((uint32_t)on));
+        : "l"(p), "r"(on));
     return x;
 }
-__device__ __forceinline__ double ld_if(const double *p, bool on)
+__device__ __forceinline__ double ld_if(const double *p, uint32_t on)
 {
     double x;
     asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t@q ld.global.nc.f64 %0, [%1];\n\t}"
         : "=d"(x)
-        : "l"(p), "r"((uint32_t)on));
+        : "l"(p), "r"(on));
     return x;
 }
 
 template <typename T, int G, int R, int M, int U, int GH> __global__ void __launch_bounds__(kGatherThreads) k_gather(GatherArgs a)
 {
-    constexpr int N = Ids<R>::n;
+    constexpr int N = Ids<R>::n, WPL = (U + G - 1) / G;   // WPL: words a lane loads of a batch
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint16_t *tab = reinterpret_cast<uint16_t *>(smem_raw);   // [k][G][N]; color 0: adds nothing
+    __shared__ uint32_t hits[R][G], seconds[R][G];            // a bit per color: some set holds it; the second does
+    uint16_t *tab = reinterpret_cast<uint16_t *>(smem_raw);   // [k][G][N]
     const int slot0 = blockIdx.y * (G * R);
+    for (int i = threadIdx.x; i < R * G; i += kGatherThreads) (&hits[0][0])[i] = (&seconds[0][0])[i] = 0;
+    __syncthreads();
     for (int i = threadIdx.x; i < a.k * G * N; i += kGatherThreads) {
         const int d = i / (G * N), l = (i - d * (G * N)) / N, r = i % N;
         const int slot = slot0 + r * G + l;
-        uint16_t x = 0xffffu;
+        uint16_t x = 0;
         if (d > 0 && r < R)
             for (int m = 0; m < M; ++m) {
                 if (slot >= a.start[m + 1] - a.start[m]) break;
                 const uint16_t y = __ldg(a.idx + (size_t)(d - 1) * a.nA + a.start[m] + slot);
-                if (y != 0xffffu) x = (uint16_t)(y | m << 13);
+                if (y == 0xffffu) continue;
+                x = (uint16_t)(M > 2 ? y | m << 13 : y);
+                atomicOr(&hits[r][l], 1u << d);
+                if (m == 1) atomicOr(&seconds[r][l], 1u << d);
             }
         tab[i] = x;
     }
@@ -438,6 +448,9 @@ template <typename T, int G, int R, int M, int U, int GH> __global__ void __laun
     __syncthreads();
     T *sacc = reinterpret_cast<T *>(rest) + threadIdx.x;   // M > 2: [R][M][threads], a thread's own
     const int lane = threadIdx.x & 31, lg = lane % G, grp = lane / G;
+    uint32_t hit[R], second[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) hit[r] = hits[r][lg], second[r] = seconds[r][lg];
     const uint16_t *mytab = tab + lg * N;
     const T *aux = reinterpret_cast<const T *>(a.aux);
     for (;;) {
@@ -446,7 +459,8 @@ template <typename T, int G, int R, int M, int U, int GH> __global__ void __laun
         t = __shfl_sync(0xffffffffu, t, 0);
         int v0, v1;
         if (!chunk_of(a.map, t, v0, v1)) break;
-        for (int v = v0 + grp; v < v1; v += 32 / G) {
+        for (int vb = v0; vb < v1; vb += 32 / G) {
+            const int v = vb + grp;
             T acc[M][R];
 #pragma unroll
             for (int m = 0; m < M; ++m)
@@ -455,28 +469,33 @@ template <typename T, int G, int R, int M, int U, int GH> __global__ void __laun
                     acc[m][r] = T(0);
                     if (M > 2) sacc[(r * M + m) * kGatherThreads] = T(0);
                 }
-            const int beg = __ldg(a.off + v), end = __ldg(a.off + v + 1);
-            uint32_t w[U];   // the next batch's neighbour words, a batch ahead
+            const int beg = v < v1 ? __ldg(a.off + v) : 0, end = v < v1 ? __ldg(a.off + v + 1) : 0;
+            const int most = __reduce_max_sync(0xffffffffu, end - beg);
+            uint32_t w[WPL];
+            auto words = [&](int e) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) w[u] = beg + u < end ? (uint32_t)__ldg(a.adjd + beg + u) : 0u;
-            for (int e = beg; e < end; e += U) {
+                for (int i = 0; i < WPL; ++i)
+                    w[i] = i * G + lg < U && e + i * G + lg < end ? (uint32_t)__ldg(a.adjd + e + i * G + lg) : 0u;
+            };
+            words(beg);
+            for (int b = 0; b < most; b += U) {
                 T x[U][R];
                 uint32_t mem[U][R];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
+                    const uint32_t z = G == 1 ? w[u % WPL] : __shfl_sync(0xffffffffu, w[u / G], lane - lg + u % G);
+                    const uint32_t bit = 1u << (z >> 28);
                     uint32_t id[(N + 1) / 2];
-                    load_ids<N>(mytab + (w[u] >> 28) * (G * N), id);
-                    const T *row = aux + (size_t)(w[u] & 0x0fffffffu) * a.pitch;
+                    load_ids<N>(mytab + (z >> 28) * (G * N), id);
+                    const T *row = aux + (size_t)(z & 0x0fffffffu) * (uint32_t)a.pitch;
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
-                        const uint32_t c = r & 1 ? id[r / 2] >> 16 : id[r / 2] & 0xffffu;
-                        x[u][r] = ld_if(row + (c & 0x1fffu), c != 0xffffu);
-                        // the member; where there is none, x is 0 and any will do
-                        mem[u][r] = M > 2 ? (c == 0xffffu ? 0u : c >> 13) : c & 0x2000u;
+                        const uint32_t c = N == 1 ? id[0] : r & 1 ? id[r / 2] >> 16 : id[r / 2] & 0xffffu;
+                        x[u][r] = ld_if(row + (M > 2 ? c & 0x1fffu : c), hit[r] & bit);
+                        mem[u][r] = M > 2 ? c >> 13 : second[r] & bit;
                     }
                 }
-#pragma unroll
-                for (int u = 0; u < U; ++u) w[u] = e + U + u < end ? (uint32_t)__ldg(a.adjd + e + U + u) : 0u;
+                words(beg + b + U);
 #pragma unroll
                 for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -491,6 +510,7 @@ template <typename T, int G, int R, int M, int U, int GH> __global__ void __laun
                         }
                     }
             }
+            if (v >= v1) continue;
             T *o = reinterpret_cast<T *>(a.out) + (size_t)v * a.out_pitch + slot0;
 #pragma unroll
             for (int m = 0; m < M; ++m)
