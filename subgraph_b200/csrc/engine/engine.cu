@@ -1795,12 +1795,13 @@ const void *rooted_table(const RunCtx &c, const rt::RootedPlan &rp, const Rooted
 // Vertices of more neighbours than this are a gather's hubs (a CTA's chain of
 // adds each) and do not share a warp's work.  Wide rows: a warp of a full SM
 // takes about 560 cycles a neighbour, and no list should outlast the work of
-// all (nnz neighbours at about 50 cycles over 148 SMs).  Narrow rows: about
-// 150 cycles a neighbour against the longest hub's 12.
-int hub_deg(const DeviceGraph &g, int nA)
+// all (nnz neighbours at about 50 cycles over 148 SMs).  Narrow rows: a share
+// of the longest list, whose chain takes as long anyway: about 12 times faster
+// a neighbour than a vertex's share of a warp, 4 times faster than the warp a
+// vertex of few slots gets.
+int hub_deg(const DeviceGraph &g, int nA, int slots)
 {
-    if (nA <= 1) return 256;
-    const int64_t d = nA > 64 ? g.nnz / 4096 : g.max_degree / 12;
+    const int64_t d = nA > 64 ? g.nnz / 4096 : g.max_degree / (slots <= 4 ? 8 : 12);
     return (int)std::min<int64_t>(8192, std::max<int64_t>(256, d));
 }
 
@@ -1871,8 +1872,8 @@ Status run_rooted(RunCtx &c, const RootedSlot &w, int32_t rows, int coloring, do
             if (root && q.main_leaf) ga.out = w.agg, ga.out_pitch = 1;
             else if (q.main_leaf) ga.out = const_cast<void *>(rooted_table(c, rp, w, rows, q.s)), ga.out_pitch = rp.tab[q.s].pitch;
             else ga.out = w.agg, ga.out_pitch = rp.agg_pitch;
-            ga.hubs = std::min(V, degree_prefix(g, hub_deg(g, q.nA) + 1));
-            ga.map = rt::make_chunks(g.h_degree, ga.hubs, V, 512, 32 / rt::gather_lanes(ga), 32);
+            ga.hubs = std::min(V, degree_prefix(g, hub_deg(g, q.nA, co.slots) + 1));
+            ga.map = rt::make_chunks(g.h_degree, ga.hubs, V, 512, ga.slots <= 4 ? 1 : 32 / rt::gather_lanes(ga), 32);
             ga.ticket = w.ticket + kStepTickets * i;
             ga.hub_ticket = ga.ticket + kStepTickets - 1;
             c.launches += rt::launch_gather(ga, c.fp64, g.sm_count, st);

@@ -459,6 +459,67 @@ template <typename T, int G, int R, int M, int U, int GH> __global__ void __laun
         t = __shfl_sync(0xffffffffu, t, 0);
         int v0, v1;
         if (!chunk_of(a.map, t, v0, v1)) break;
+        if constexpr (R == 1 && G <= 4) {
+            // long lists of few slots: a warp a vertex, the groups of G lanes each
+            // fetch a neighbour, DEP batches ahead, and every group adds all of them in
+            // order (by shuffles).  Eight vertices a warp left lists of 3000 neighbours
+            // with eight in flight: 0.29 ms at 12 M entries and four slots, now 0.18.
+            // At eight slots of three sets the adds cost more than the wait (0.9 ->
+            // 1.2 ms at 31 M entries).
+            if (__ldg(a.off + v0 + 1) - __ldg(a.off + v0) >= (G == 1 ? 32 : 128)) {
+                constexpr int NPF = 32 / G, DEP = G == 1 ? 3 : 6;
+                for (int v = v0; v < v1; ++v) {
+                    const int beg = __ldg(a.off + v), end = __ldg(a.off + v + 1);
+                    auto word = [&](int e) { return e + grp < end ? (uint32_t)__ldg(a.adjd + e + grp) : 0u; };
+                    T x[DEP], acc[M];
+                    uint32_t mem[DEP], z[DEP];
+                    auto fetch = [&](int q, uint32_t y) {
+                        const uint32_t bit = 1u << (y >> 28), c = mytab[(y >> 28) * G];
+                        x[q] = ld_if(aux + (size_t)(y & 0x0fffffffu) * (uint32_t)a.pitch + (M > 2 ? c & 0x1fffu : c), hit[0] & bit);
+                        mem[q] = M > 2 ? c >> 13 : second[0] & bit;
+                    };
+#pragma unroll
+                    for (int m = 0; m < M; ++m) acc[m] = T(0);
+#pragma unroll
+                    for (int q = 0; q < DEP; ++q) z[q] = word(beg + q * NPF);
+#pragma unroll
+                    for (int q = 0; q < DEP; ++q) {
+                        fetch(q, z[q]);
+                        z[q] = word(beg + (DEP + q) * NPF);
+                    }
+                    for (int e = beg; e < end; e += DEP * NPF) {
+#pragma unroll
+                        for (int q = 0; q < DEP; ++q) {
+                            if (e + q * NPF >= end) break;
+#pragma unroll
+                            for (int i = 0; i < NPF; ++i) {
+                                const T y = __shfl_sync(0xffffffffu, x[q], i * G + lg);
+                                if constexpr (M == 1) {
+                                    acc[0] = add_rn(acc[0], y);
+                                } else {
+                                    const uint32_t who = __shfl_sync(0xffffffffu, mem[q], i * G + lg);
+                                    if constexpr (M == 2) {
+                                        add_one_of(acc[0], acc[1], y, who);
+                                    } else {
+#pragma unroll
+                                        for (int m = 0; m < M; ++m) add_if(acc[m], y, who == (uint32_t)m);
+                                    }
+                                }
+                            }
+                            fetch(q, z[q]);
+                            z[q] = word(e + (2 * DEP + q) * NPF);
+                        }
+                    }
+                    if (grp == 0) {
+#pragma unroll
+                        for (int m = 0; m < M; ++m)
+                            if (slot0 + lg < a.start[m + 1] - a.start[m])
+                                reinterpret_cast<T *>(a.out)[(size_t)v * a.out_pitch + slot0 + a.start[m] + lg] = acc[m];
+                    }
+                }
+                continue;
+            }
+        }
         for (int vb = v0; vb < v1; vb += 32 / G) {
             const int v = vb + grp;
             T acc[M][R];
