@@ -12,8 +12,9 @@ tables, 16 colorings per step (coloring c seeded srand(7 + c)).
             built from pinned host CSC arrays (H2D copy inside the timed
             region), all colorings counted, raw counts read back (D2H);
             W untimed warm-up steps first, as for value.
-  roofline  the fused aggregation+eMA kernel: compulsory bytes per launch
-            divided by its CUDA-event duration, against MEASURED_PEAKS.json.
+  roofline  the dominant step (gather and product kernels of one
+            sub-template): compulsory bytes divided by its CUDA-event
+            duration, against MEASURED_PEAKS.json.
   cpu_baseline  the reference's own CPU code (its CountMat::colorCounting,
             built from the reference sources into oracle/_ref/) on the host
             cores, on the first two colorings the GPU timed, same graph: its
@@ -51,13 +52,7 @@ TEMPLATES = {
 }
 WORKLOADS = {
     # the 12-vertex tree on R-MAT scale 20, edge factor 8: 16 colorings per step
-    "tree12_rmat20_ef8": dict(scale=20, ef=8, template="tree12", per_step=16, seed=7,
-                              # DRAM bytes (read + write) of one launch of the dominant stage (sub 10),
-                              # measured by ncu on the same kernel at R-MAT scale 18 (tree12_rmat18_ef8)
-                              # and scaled by the ratio of its algorithmic bytes (x4.0006)
-                              dominant_traffic=dict(sub=10, bytes=2.5298e9 * 4.0006,
-                                                    source="ncu dram__bytes_read.sum + dram__bytes_write.sum of "
-                                                           "the sub-10 launch at R-MAT scale 18, x4.0006 to scale 20")),
+    "tree12_rmat20_ef8": dict(scale=20, ef=8, template="tree12", per_step=16, seed=7),
     "p3_rmat16_ef16": dict(scale=16, ef=16, template="p3", per_step=1, seed=7),
     "tree5_rmat20_ef6": dict(scale=20, ef=6, template="tree5", per_step=10, seed=7),
     "spider7_rmat21_ef8": dict(scale=21, ef=8, template="spider7", per_step=64, seed=7),
@@ -443,9 +438,9 @@ def main():
     def seeds(step):  # rank-disjoint colorings
         return w["seed"] + (step * world + rank) * B
 
-    # warm-up; the first call on a new graph also times the tile-shape
-    # candidates of every stage shape (the autotuner): its wall time against
-    # the second call's is the tuning cost
+    # warm-up; the first call on a new graph also allocates its tables and, in
+    # the forms that tune (the persistent queue), times the tile shapes: its
+    # wall time against the second call's is that cost
     warm_ms = []
     for s in range(args.warmup):
         torch.cuda.synchronize()
@@ -536,17 +531,14 @@ def main():
     # the dominant kernel: the sub-template stage whose fused launches take the most time
     achieved = top["bytes"] / (top["ms"] / 1000.0) / 1e9 if top["ms"] > 0 else 0.0
     all_achieved = fused_bytes / (fused_ms / 1000.0) / 1e9 if fused_ms > 0 else 0.0
-    dt = w.get("dominant_traffic")
-    traffic = dt["bytes"] if dt and dt["sub"] == top["sub"] and args.batch == 0 else None
     line = {
         "metric": METRIC, "value": value, "unit": "colorings/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "fp32", "data": "synthetic", "config": config_of(args, w),
         "rel_err_vs_fp64": err,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak if peak else 0.0, "peak_kind": peak_kind, "traffic": traffic,
-                     "traffic_source": dt["source"] if traffic else None,
-                     "kernel": f"fused aggregation + eMA of sub {top['sub']} (the dominant stage)",
+                     "frac": achieved / peak if peak else 0.0, "peak_kind": peak_kind, "traffic": None,
+                     "kernel": f"gather and product step of sub {top['sub']} (the dominant step)",
                      "launch_ms": top["ms"] / max(top["launches"], 1),
                      "alg_bytes_per_launch": top["bytes"] / max(top["launches"], 1),
                      "all_fused": {"achieved": all_achieved, "frac": all_achieved / peak if peak else 0.0,
@@ -558,9 +550,8 @@ def main():
         "gpu_launches": launches,
         "clocks": clocks,
         "autotune": {"first_call_ms": first_ms, "second_call_ms": steady_ms,
-                     "note": "wall clock of the first two warm-up steps: the first call on a new graph times "
-                             "the tile-shape candidates of each stage shape; later calls (the timed steps and "
-                             "the e2e leg, whose per-step graphs have the same signature) reuse the choice"},
+                     "note": "wall clock of the first two warm-up steps: the first call on a new graph allocates its "
+                             "tables; only the persistent queue times tile shapes"},
     }
     if forms:
         line["forms"] = forms

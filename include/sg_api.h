@@ -161,11 +161,14 @@ typedef struct {
     uint32_t seed_base;     /* coloring c uses srand(seed_base + c) */
     int32_t mode;           /* SG_MODE_* */
     int32_t batch;          /* > 0: colorings per batch (batched form); 0: plain */
-    int32_t hub_threshold;  /* degree above which aggregation is chunked; 0 = never
-                               (exact reference arithmetic for every vertex) */
+    int32_t hub_threshold;  /* general path and persistent form: degree above which a
+                               vertex is aggregated by itself, in the persistent form in
+                               chunks; 0 = never (the default form decides for itself
+                               and always sums in the reference's order) */
     int32_t profile;        /* != 0: time every fused launch with CUDA events */
-    int32_t no_autotune;    /* != 0: use the default tile shapes instead of timing the
-                               candidates of each new stage shape once per graph */
+    int32_t no_autotune;    /* != 0: general path and persistent form: use the default tile
+                               shapes instead of timing the candidates of each new stage
+                               shape once per graph (the default form times nothing) */
     int32_t exact;          /* != 0: the reference's FP32 operations in the reference's
                                order for every vertex and product (no fused multiply-add,
                                no hub chunking): per-vertex values bit-identical to the
@@ -175,11 +178,17 @@ typedef struct {
                                sums them in chunks unless exact is set */
     int32_t wait_limit_ms;  /* batched form: how long a work item may wait for its inputs
                                before the call fails with SG_ERR_TIMEOUT (0 = 2000 ms) */
+                            /* Any of no_blocked, no_rooted and no_flat set selects the
+                               general path (full-width tables) without that form; the
+                               default form keeps rooted rows (the color sets with the
+                               vertex's color); all give identical values */
     int32_t no_blocked;     /* 1: no register-blocked eMA (every output computed by its
                                own split loop); the two forms give identical values */
     int32_t persistent;     /* batched form: 1 = one persistent work-queue launch per batch
-                               (colorings in separate table slots); 0 = interleaved groups
-                               (the batch's colorings share table rows and neighbour passes) */
+                               (colorings in separate table slots); 0 = up to four colorings
+                               in flight on streams of their own, on the general path
+                               interleaved groups (the batch's colorings share table rows
+                               and neighbour passes) */
     int32_t no_rooted;      /* 1: no rooted form of the register-blocked eMA (a vertex of color c
                                computes only the outputs and products whose sets hold c, over
                                the other k-1 colors); the two give identical values */

@@ -1974,8 +1974,9 @@ Status make_streams(GraphState &gs, int n)
     return Status::ok();
 }
 
-// Slots for up to `want` colorings in flight that fit the free memory.
-Status rooted_admit(const DeviceGraph &g, const Workspace &w, const RootedSizes &z, int want, int &slots)
+// Slots for up to `want` colorings in flight that take no more than `share` of
+// the free memory.
+Status rooted_admit(const DeviceGraph &g, const Workspace &w, const RootedSizes &z, int want, double share, int &slots)
 {
     slots = std::max(1, want);
     if (slots == 1) return Status::ok();
@@ -1988,7 +1989,7 @@ Status rooted_admit(const DeviceGraph &g, const Workspace &w, const RootedSizes 
     SG_CK(cudaMemGetInfo(&free_b, &total_b));
     const size_t per = z.all() + (size_t)g.V + 8 * ((size_t)g.V / 8 + 2) + 8 * (size_t)g.V1;
     const size_t have = w.arena_bytes + w.agg_bytes + w.cnt_bytes + w.scnt_bytes + w.adjc_bytes;
-    while (slots > 1 && per * (size_t)slots > (size_t)((double)(free_b + have) * 0.85)) --slots;
+    while (slots > 1 && per * (size_t)slots > (size_t)((double)(free_b + have) * share)) --slots;
     return Status::ok();
 }
 
@@ -1999,12 +2000,15 @@ Status count_rooted(RunCtx &c, const CountOptions &o, double *raw, CountStats *s
     cudaStream_t st = g.stream;
     const RootedSizes z = rooted_sizes(g, c.re->plan[c.fp64], g.V2, c.es);
     // several colorings in flight: the chains of one's hubs run beside the
-    // others' work (profiled launches one after another)
+    // others' work (profiled launches one after another); a quarter of the
+    // memory at most, one coloring where more cannot be had
     int S = 1;
     const int most = o.batch > 0 ? std::min(o.batch, kRootedStreams) : kRootedStreams;
-    SG_CKS(rooted_admit(g, w, z, c.profile ? 1 : std::min(o.n_colorings, most), S));
+    SG_CKS(rooted_admit(g, w, z, c.profile ? 1 : std::min(o.n_colorings, most), 0.25, S));
     std::vector<RootedSlot> slot;
-    SG_CKS(rooted_reserve(g, w, z, S, o.n_colorings, slot));
+    Status room = rooted_reserve(g, w, z, S, o.n_colorings, slot);
+    if (room.code == 2 && S > 1) room = rooted_reserve(g, w, z, S = 1, o.n_colorings, slot);
+    SG_CKS(room);
     std::vector<uint32_t> seeds(o.n_colorings);
     for (int i = 0; i < o.n_colorings; ++i) seeds[i] = o.seed_base + (uint32_t)i;
     SG_CKS(upload_seeds(g, w, seeds));
@@ -2606,7 +2610,7 @@ static Status count_jobs_rooted(DeviceGraph &g, std::vector<RunCtx> &ctx, const 
     RootedSizes z;
     for (RunCtx &c : ctx) z.cover(rooted_sizes(g, c.re->plan[c.fp64], g.V2, c.es));
     int S = 1;
-    SG_CKS(rooted_admit(g, w, z, std::min(o.batch > 0 ? o.batch : 8, n), S));
+    SG_CKS(rooted_admit(g, w, z, std::min(o.batch > 0 ? o.batch : 8, n), 0.85, S));
     std::vector<RootedSlot> slot;
     SG_CKS(rooted_reserve(g, w, z, S, n, slot));
     SG_CKS(upload_seeds(g, w, std::vector<uint32_t>(seeds, seeds + n)));
