@@ -1873,7 +1873,12 @@ Status run_rooted(RunCtx &c, const RootedSlot &w, int32_t rows, int coloring, do
             else if (q.main_leaf) ga.out = const_cast<void *>(rooted_table(c, rp, w, rows, q.s)), ga.out_pitch = rp.tab[q.s].pitch;
             else ga.out = w.agg, ga.out_pitch = rp.agg_pitch;
             ga.hubs = std::min(V, degree_prefix(g, hub_deg(g, q.nA, co.slots) + 1));
-            ga.map = rt::make_chunks(g.h_degree, ga.hubs, V, 512, ga.slots <= 4 ? 1 : 32 / rt::gather_lanes(ga), 32);
+            // a warp's chunk: 512 entries, fewer where the graph would not give every
+            // warp of the device four of them (0.8 M entries: 236 CTAs of 740)
+            const int entries = (int)std::min<int64_t>(512, std::max<int64_t>(64, g.nnz / (g.sm_count * 128)));
+            // (a warp to a vertex of a long list: k_gather's rule)
+            ga.map = rt::make_chunks(g.h_degree, ga.hubs, V, entries, 32 / rt::gather_lanes(ga),
+                                     ga.slots <= 1 ? 32 : ga.slots <= 4 ? 128 : 1 << 30, 32);
             ga.ticket = w.ticket + kStepTickets * i;
             ga.hub_ticket = ga.ticket + kStepTickets - 1;
             c.launches += rt::launch_gather(ga, c.fp64, g.sm_count, st);
@@ -2025,6 +2030,9 @@ Status count_rooted(RunCtx &c, const CountOptions &o, double *raw, CountStats *s
     if (S > 1) join_streams(c.gs, S, st);
     if (status.code) {
         cudaStreamSynchronize(st);
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        ev_sum(c.fused_ev);
         return status;
     }
     SG_CK(cudaEventRecord(e1, st));

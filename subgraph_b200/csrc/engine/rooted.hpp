@@ -165,7 +165,9 @@ cudaError_t upload_rooted_tables(const Plan &p, const RootedPlan &rp, RootedTabl
 // blocks of an index structure (engine.cu): the register-blocked schedule
 bool rooted_blocks(int k, int n, int pm, std::vector<int32_t> &rows, int &nblocks, int &shape);
 
-ChunkMap make_chunks(const std::vector<int32_t> &degree, int32_t first, int32_t last, int target, int least,
+// chunks of about `target` entries, at least `least` vertices each (one where a
+// vertex has `alone` neighbours or more, a power of two), at most `most`
+ChunkMap make_chunks(const std::vector<int32_t> &degree, int32_t first, int32_t last, int target, int least, int alone,
                      int most);
 
 }  // namespace rt

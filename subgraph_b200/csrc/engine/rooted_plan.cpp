@@ -261,7 +261,8 @@ cudaError_t upload_rooted_tables(const Plan &p, const RootedPlan &rp, RootedTabl
     return cudaSuccess;
 }
 
-ChunkMap make_chunks(const std::vector<int32_t> &degree, int32_t first, int32_t last, int target, int least, int most)
+ChunkMap make_chunks(const std::vector<int32_t> &degree, int32_t first, int32_t last, int target, int least, int alone,
+                     int most)
 {
     ChunkMap m{};
     int32_t v = first;
@@ -274,7 +275,7 @@ ChunkMap make_chunks(const std::vector<int32_t> &degree, int32_t first, int32_t 
             (int32_t)(std::partition_point(degree.begin() + v, degree.begin() + last, [&](int32_t d) { return d >= lo; }) -
                       degree.begin());
         m.first[m.n] = v;
-        m.per[m.n] = std::min(most, std::max(least, target >> c));
+        m.per[m.n] = std::min(most, std::max((1 << c) >= alone ? 1 : least, target >> c));
         m.base[m.n + 1] = m.base[m.n] + (end - v + m.per[m.n] - 1) / m.per[m.n];
         ++m.n;
         m.first[m.n] = end;
