@@ -24,7 +24,7 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-r
 CXX_FLAGS = ["-std=c++17", "-O3", "-fPIC", "-Wall", "-Wno-unused-function"]
 
 HOST_SOURCES = ["host/graph_io.cpp", "host/plan.cpp", "capi.cpp", "engine/rooted_plan.cpp"]
-CUDA_SOURCES = ["engine/kernels.cu", "engine/blocked.cu", "engine/blocked_a.cu", "engine/blocked_b.cu",
+CUDA_SOURCES = ["engine/launch.cu", "engine/kernels.cu", "engine/blocked.cu", "engine/blocked_a.cu", "engine/blocked_b.cu",
                 "engine/blocked_c.cu", "engine/blocked_d.cu", "engine/blocked_e.cu", "engine/engine.cu", "engine/batch.cu", "engine/noalloc.cu",
                 "engine/input_gpu.cu",
                 "engine/rooted.cu", "engine/rooted_gather_f32.cu", "engine/rooted_gather_f64.cu", "engine/rooted_ema.cu", "engine/rooted_ema_a.cu", "engine/rooted_ema_b.cu",

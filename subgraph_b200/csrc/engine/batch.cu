@@ -11,6 +11,7 @@
 // then returns at once and the host reports SG_ERR_TIMEOUT).  Tables produced
 // inside the launch are read through L2 (fused_tile<..., COH = true>).
 #include "kernels.cuh"
+#include "launch.hpp"
 #include "tile.cuh"
 
 namespace sg {
@@ -135,13 +136,9 @@ cudaError_t launch_persistent(const BatchStage *stages, int nstages, int total_i
                               unsigned long long *stage_end)
 {
     auto go = [&](auto kern) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         // every resident CTA claims items (a claimed item only waits for items
         // claimed earlier by running CTAs, so residency needs no guarantee)
-        int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBatchThreads, smem) != cudaSuccess ||
-            per_sm < 1)
-            per_sm = 1;
+        const int per_sm = resident_ctas((const void *)kern, kBatchThreads, smem);
         kern<<<sm_count * per_sm, kBatchThreads, smem, st>>>(stages, nstages, total_items, done, ctl, wait_cycles,
                                                                stage_end);
     };

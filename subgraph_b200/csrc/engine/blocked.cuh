@@ -6,6 +6,7 @@
 // (blocked_a.cu ... blocked_e.cu) that compile in parallel.
 #pragma once
 #include "kernels.cuh"
+#include "launch.hpp"
 #include "tile.cuh"
 
 namespace sg {
@@ -41,10 +42,7 @@ template <int NT, int N, int P>
 static void launch_blk_q(const StageDesc &d, const FusedConfig &cfg, cudaStream_t st)
 {
     auto go = [&](auto kern) {
-        if (cfg.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem);
-        int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, cfg.smem) != cudaSuccess || per_sm < 1)
-            per_sm = 1;
+        const int per_sm = resident_ctas((const void *)kern, NT, cfg.smem);
         const int grid = std::max(1, std::min(d.ntiles - d.tile_begin, cfg.grid * per_sm));
         if (d.ticket) cudaMemsetAsync(d.ticket, 0, sizeof(int32_t), st);
         kern<<<grid, NT, cfg.smem, st>>>(d);

@@ -9,6 +9,7 @@
 // CPU arithmetic (CSCGraph.hpp:242-307, DataTableColMajor.cpp:346-400) bit
 // for bit.
 #include "kernels.cuh"
+#include "launch.hpp"
 
 #include <algorithm>
 #include <cstdio>
@@ -196,10 +197,7 @@ static void launch_hub_exact_v(const HubArgs &h, int sm_count, cudaStream_t st)
     constexpr size_t smem = (size_t)W * hub_warp_bytes<T, NSLOT, BR>();
     static_assert(smem <= 227 * 1024, "a CTA's rings must fit shared memory");
     auto kern = k_hub_exact<T, W, NSLOT, BR>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * W, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
+    const int per_sm = resident_ctas((const void *)kern, 32 * W, smem);
     const int grid = std::max(1, std::min((items + W - 1) / W, sm_count * per_sm));
     cudaMemsetAsync(h.ticket, 0, sizeof(int32_t), st);
     kern<<<grid, 32 * W, smem, st>>>(h);
@@ -449,10 +447,7 @@ template <typename T, int NT>
 static void launch_fused_q(const StageDesc &d, const FusedConfig &cfg, cudaStream_t st)
 {
     auto go = [&](auto kern) {
-        if (cfg.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem);
-        int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, cfg.smem) != cudaSuccess || per_sm < 1)
-            per_sm = 1;
+        const int per_sm = resident_ctas((const void *)kern, NT, cfg.smem);
         const int grid = std::max(1, std::min(d.ntiles - d.tile_begin, cfg.grid * per_sm));
         if (d.ticket) cudaMemsetAsync(d.ticket, 0, sizeof(int32_t), st);
         kern<<<grid, NT, cfg.smem, st>>>(d);

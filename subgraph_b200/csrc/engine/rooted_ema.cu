@@ -103,8 +103,9 @@ void launch_ema(const EmaArgs &a0, bool fp64, cudaStream_t st)
     const size_t smem = ema_smem(a.nA, a.nM, a.nO, a.tile_v, fp64 ? 8 : 4, a.is_root);
     const int tiles = (a.V + a.tile_v - 1) / a.tile_v;
     auto go = [&](auto kern) {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<tiles, a.is_root ? 128 : ema_threads(smem), smem, st>>>(a);
+        const int threads = a.is_root ? 128 : ema_threads(smem);
+        resident_ctas((const void *)kern, threads, smem);
+        kern<<<tiles, threads, smem, st>>>(a);
     };
     if (fp64) go(k_ema<double, false>);
     else if (a.fused) go(k_ema<float, true>);

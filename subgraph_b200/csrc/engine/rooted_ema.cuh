@@ -6,6 +6,7 @@
 // one index structure (|s|-1 vertices, mains of |main|-1, over k-1 colors)
 // serves every vertex; results go back to the relative columns.
 #pragma once
+#include "launch.hpp"
 #include "rooted.hpp"
 #include "tile.cuh"
 
@@ -74,7 +75,7 @@ template <int N, int P> __global__ void __launch_bounds__(kEmaThreads) k_ema_blk
 template <int N, int P> static void launch_ema_shape(const EmaArgs &a, size_t smem, cudaStream_t st)
 {
     auto kern = k_ema_blk<N, P>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    resident_ctas((const void *)kern, ema_threads(smem), smem);
     kern<<<(a.V + a.tile_v - 1) / a.tile_v, ema_threads(smem), smem, st>>>(a);
 }
 

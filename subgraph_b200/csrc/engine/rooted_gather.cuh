@@ -2,8 +2,8 @@
 // and FP64 tables in rooted_gather_f32.cu and rooted_gather_f64.cu.
 #pragma once
 #include <algorithm>
-#include <atomic>
 
+#include "launch.hpp"
 #include "rooted.hpp"
 #include "tile.cuh"
 
@@ -585,22 +585,6 @@ template <typename T, int G, int R, int M, int U, int GH> __global__ void __laun
 
 namespace {
 
-// CTAs of a kernel an SM holds; the answer for the last (device, size) is kept
-// a kernel (the driver's takes microseconds).
-template <typename F> int resident(F kern, size_t smem, std::atomic<uint64_t> &last)
-{
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t key = (uint64_t)dev << 40 | (uint64_t)smem << 8, got = last.load(std::memory_order_relaxed);
-    if ((got & ~(uint64_t)0xff) == key && (got & 0xff)) return (int)(got & 0xff);
-    // static shared memory counts against the default limit too
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kGatherThreads, smem) != cudaSuccess || n < 1) n = 1;
-    last.store(key | (uint64_t)std::min(n, 255), std::memory_order_relaxed);
-    return n;
-}
-
 int gather_grid(const GatherArgs &a, int per_sm, int sm_count, int hub_cols)
 {
     const int64_t items = (int64_t)a.hubs * ((a.nA + hub_cols - 1) / hub_cols);
@@ -613,8 +597,7 @@ template <typename T, int G, int R, int M, int U, int GH> void go_narrow_h(const
     const size_t sacc = M > 2 ? (size_t)R * M * kGatherThreads * sizeof(T) : 0;
     const size_t smem = ((size_t)a.k * G * Ids<R>::n * 2 + 15) / 16 * 16 + std::max(sacc, a.hubs > 0 ? hub_bytes<T, GH>() : 0);
     auto kern = k_gather<T, G, R, M, U, GH>;
-    static std::atomic<uint64_t> last{0};
-    const int per_sm = resident(kern, smem, last);
+    const int per_sm = resident_ctas((const void *)kern, kGatherThreads, smem);
     kern<<<dim3(gather_grid(a, per_sm, sm_count, GH), (a.slots + G * R - 1) / (G * R)), kGatherThreads, smem, st>>>(a);
 }
 
@@ -659,8 +642,7 @@ template <typename T, int R, int M, int RR, int BR, int NP> void go_wide_n(const
 {
     const size_t smem = wide_smem<T>(a, wide_ids<R>());
     auto kern = k_gather_wide<T, R, M, RR, BR, NP>;
-    static std::atomic<uint64_t> last{0};
-    const int per_sm = resident(kern, smem, last);
+    const int per_sm = resident_ctas((const void *)kern, kGatherThreads, smem);
     kern<<<dim3(gather_grid(a, per_sm, sm_count, 32), (a.slots + 32 * R - 1) / (32 * R)), kGatherThreads, smem, st>>>(a);
 }
 
