@@ -85,6 +85,20 @@ Poly poly_xpow(uint64_t n)
 
 int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
+// One rooted coloring in flight.  Every coloring has buffers of its own, so that
+// the device's pool finds them again for the next graph of the same size
+// (neighbours for four colorings in one block made it remap memory between
+// that block and the upload's buffers, at up to 0.8 s a graph), and so that
+// colorings can be given up one by one where memory is short.
+struct RootedMem {
+    void *tables = nullptr;            // arena, aggregates, neighbour counts, scaled counts
+    size_t tables_bytes = 0;
+    int32_t *adjd = nullptr;           // [nnz] neighbour id | relative color << 28
+    size_t adjd_bytes = 0;
+    void *small = nullptr;             // counters, root partials, root values, colors
+    size_t small_bytes = 0;
+};
+
 // Device buffers reused across count() calls on one graph.
 struct Workspace {
     void *arena = nullptr;
@@ -112,17 +126,9 @@ struct Workspace {
     int32_t *tile_ticket = nullptr;    // fused kernels' tile counters, one per concurrent stream
     size_t tile_ticket_bytes = 0;
     uint64_t generation = 0;   // bumped whenever a buffer above is re-allocated
-    // rooted rows: aggregates, neighbour counts and their scaled copy, counters
-    void *agg = nullptr;
-    size_t agg_bytes = 0;
-    void *cnt = nullptr;
-    size_t cnt_bytes = 0;
-    void *scnt = nullptr;
-    size_t scnt_bytes = 0;
-    double *root = nullptr;            // root values of a main that is not one-hot
-    size_t root_bytes = 0;
-    int32_t *rticket = nullptr;
-    size_t rticket_bytes = 0;
+    // rooted rows: the memory of the colorings in flight.  The first one's
+    // tables and neighbours are `arena` and `adjc`
+    std::vector<RootedMem> rooted;
 };
 
 struct DevicePlanTables {
@@ -247,6 +253,27 @@ void keep_pool_memory(int device)
     }
 }
 
+size_t pool_unused(int device)
+{
+    cudaMemPool_t pool;
+    uint64_t reserved = 0, used = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+        return 0;
+    return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
+// Memory a call can still have: the driver's free memory and what the device's
+// pool holds unused.
+Status available_bytes(int device, size_t &bytes)
+{
+    size_t free_b = 0, total_b = 0;
+    SG_CK(cudaMemGetInfo(&free_b, &total_b));
+    bytes = free_b + pool_unused(device);
+    return Status::ok();
+}
+
 uint64_t g_grow_count = 0;   // re-allocations so far (the workspace generation)
 
 Status grow(void **p, size_t *have, size_t need, cudaStream_t st)
@@ -266,6 +293,15 @@ Status grow(void **p, size_t *have, size_t need, cudaStream_t st)
     return Status::ok();
 }
 template <typename T> Status growT(T **p, size_t *have, size_t need, cudaStream_t st) { return grow((void **)p, have, need, st); }
+
+// The buffers of the rooted colorings `first` and later, back to the pool.
+void release_rooted(Workspace &w, size_t first, cudaStream_t st)
+{
+    for (size_t i = first; i < w.rooted.size(); ++i)
+        for (void *p : {w.rooted[i].tables, (void *)w.rooted[i].adjd, w.rooted[i].small})
+            if (p) cudaFreeAsync(p, st);
+    if (first < w.rooted.size()) w.rooted.resize(first);
+}
 
 // Register-blocked eMA tables of sub s: the output color sets (|s| colors out
 // of k) partitioned greedily into blocks U of |s|+1 colors, each block the
@@ -656,23 +692,25 @@ DeviceGraph::~DeviceGraph()
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(device);
+    GraphState state;
     {
         std::lock_guard<std::mutex> lk(g_state_mu);
         auto it = g_state.find(this);
         if (it != g_state.end()) {
-            Workspace &w = it->second.ws;
-            for (void *p : {w.arena, (void *)w.colors, (void *)w.partial, (void *)w.raw, (void *)w.windows, w.hub_partial,
-                            (void *)w.chunk_start, (void *)w.root_vertex, (void *)w.adjc, (void *)w.orig_buf,
-                            (void *)w.hub_ticket, (void *)w.tile_ticket, w.agg, w.cnt, w.scnt, (void *)w.root, (void *)w.rticket})
-                if (p) cudaFreeAsync(p, stream);
-            for (auto &kv : it->second.batches) free_batch(kv.second, stream);
-            for (cudaStream_t js : it->second.streams) {
-                cudaStreamSynchronize(js);
-                cudaStreamDestroy(js);
-            }
-
+            state = std::move(it->second);
             g_state.erase(it);
         }
+    }
+    Workspace &w = state.ws;
+    for (void *p : {w.arena, (void *)w.colors, (void *)w.partial, (void *)w.raw, (void *)w.windows, w.hub_partial,
+                    (void *)w.chunk_start, (void *)w.root_vertex, (void *)w.adjc, (void *)w.orig_buf,
+                    (void *)w.hub_ticket, (void *)w.tile_ticket})
+        if (p) cudaFreeAsync(p, stream);
+    release_rooted(w, 0, stream);
+    for (auto &kv : state.batches) free_batch(kv.second, stream);
+    for (cudaStream_t js : state.streams) {
+        cudaStreamSynchronize(js);
+        cudaStreamDestroy(js);
     }
     for (void *p : {(void *)d_off, (void *)d_adj, (void *)d_perm, (void *)d_iperm, (void *)d_jump, (void *)d_coef})
         if (p) cudaFreeAsync(p, stream);
@@ -1570,8 +1608,8 @@ Status count_batched(RunCtx &c, const CountOptions &o, double *raw, CountStats *
     int slots = std::min(o.batch, o.n_colorings);
     {
         // admission: a slot needs its table arena, colors, root partials and hub rows
-        size_t free_b = 0, total_b = 0;
-        SG_CK(cudaMemGetInfo(&free_b, &total_b));
+        size_t free_b = 0;
+        SG_CKS(available_bytes(g.device, free_b));
         const size_t held = c.gs.ws.arena_bytes;   // reused by the batch
         const size_t per_slot = (size_t)p.arena_units * V * c.es + V + 8 * (V / 8 + 2) +
                                 (size_t)c.hubs.total_chunks * (size_t)std::max(c.hub_pitch, 4) * c.es *
@@ -1737,8 +1775,8 @@ constexpr int kStepTickets = 64, kRootedTickets = 16 * kStepTickets;
 
 // Per-slot bytes of a plan whose tables have `rows` rows.
 struct RootedSizes {
-    size_t arena = 0, agg = 0, cnt = 0, scnt = 0, adjd = 0;
-    size_t all() const { return arena + agg + cnt + scnt + adjd; }
+    size_t arena = 0, agg = 0, cnt = 0, scnt = 0, adjd = 0, small = 0;
+    size_t tables() const { return arena + agg + cnt + scnt; }
     void cover(const RootedSizes &o)
     {
         arena = std::max(arena, o.arena);
@@ -1746,41 +1784,99 @@ struct RootedSizes {
         cnt = std::max(cnt, o.cnt);
         scnt = std::max(scnt, o.scnt);
         adjd = std::max(adjd, o.adjd);
+        small = std::max(small, o.small);
     }
 };
+size_t up256(size_t x) { return (x + 255) / 256 * 256; }
+// parts of a slot's small buffer: [counters][root partials][root values][colors]
+size_t small_partial() { return up256(4 * (size_t)kRootedTickets); }
+size_t small_root(const DeviceGraph &g) { return small_partial() + up256(8 * ((size_t)g.V / 8 + 2)); }
+size_t small_color(const DeviceGraph &g) { return small_root(g) + up256(8 * (size_t)g.V1); }
 RootedSizes rooted_sizes(const DeviceGraph &g, const rt::RootedPlan &rp, int32_t rows, size_t es)
 {
-    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
     RootedSizes z;
-    z.arena = up((size_t)rp.arena_units * rows * es);
-    z.agg = up(std::max((size_t)rp.agg_pitch * rows, (size_t)g.V1) * es);
-    z.cnt = up((size_t)rp.cnt_pitch * g.V1 * es);
+    z.arena = up256((size_t)rp.arena_units * rows * es);
+    z.agg = up256(std::max((size_t)rp.agg_pitch * rows, (size_t)g.V1) * es);
+    z.cnt = up256((size_t)rp.cnt_pitch * g.V1 * es);
     z.scnt = rp.need_scaled ? z.cnt : 0;
-    z.adjd = rp.need_edges ? up(4 * (size_t)g.nnz) : 0;
+    z.adjd = rp.need_edges ? up256(4 * (size_t)g.nnz) : 0;
+    z.small = small_color(g) + up256((size_t)g.V);
     return z;
 }
 
-Status rooted_reserve(DeviceGraph &g, Workspace &w, const RootedSizes &z, int slots, int ncolorings, std::vector<RootedSlot> &out)
+// The three buffers of slot i, with their sizes; slot 0 shares the general
+// path's arena and neighbours.
+struct RootedBuffers {
+    void **tables;
+    size_t *tables_bytes;
+    int32_t **adjd;
+    size_t *adjd_bytes;
+    void **small;
+    size_t *small_bytes;
+};
+RootedBuffers rooted_buffers(Workspace &w, size_t i)
+{
+    if (w.rooted.size() <= i) w.rooted.resize(i + 1);
+    RootedMem &m = w.rooted[i];
+    if (i == 0) return {&w.arena, &w.arena_bytes, &w.adjc, &w.adjc_bytes, &m.small, &m.small_bytes};
+    return {&m.tables, &m.tables_bytes, &m.adjd, &m.adjd_bytes, &m.small, &m.small_bytes};
+}
+
+Status rooted_grow(DeviceGraph &g, Workspace &w, const RootedSizes &z, size_t i, RootedSlot &out)
+{
+    const RootedBuffers b = rooted_buffers(w, i);
+    SG_CKS(grow(b.tables, b.tables_bytes, std::max<size_t>(16, z.tables()), g.stream));
+    SG_CKS(growT(b.adjd, b.adjd_bytes, z.adjd, g.stream));
+    SG_CKS(grow(b.small, b.small_bytes, z.small, g.stream));
+    char *t = (char *)*b.tables, *s = (char *)*b.small;
+    out = {t, t + z.arena, t + z.arena + z.agg, t + z.arena + z.agg + z.cnt, *b.adjd, (uint8_t *)(s + small_color(g)),
+           (double *)(s + small_partial()), (double *)(s + small_root(g)), (int32_t *)s};
+    return Status::ok();
+}
+
+// Slots for up to `want` colorings in flight.  Past the first, slots take no
+// more new memory than the device's pool holds unused, or than `share` of all
+// that is free, and no more than there is: fewer where an allocation fails.
+Status rooted_reserve(DeviceGraph &g, Workspace &w, const RootedSizes &z, int want, double share, int ncolorings,
+                      std::vector<RootedSlot> &out)
 {
     cudaStream_t st = g.stream;
-    const size_t V = (size_t)g.V, n = (size_t)slots;
-    auto some = [](size_t x) { return std::max<size_t>(16, x); };
-    SG_CKS(grow(&w.arena, &w.arena_bytes, some(z.arena * n), st));
-    SG_CKS(grow(&w.agg, &w.agg_bytes, some(z.agg * n), st));
-    SG_CKS(grow(&w.cnt, &w.cnt_bytes, some(z.cnt * n), st));
-    SG_CKS(grow(&w.scnt, &w.scnt_bytes, some(z.scnt * n), st));
-    SG_CKS(growT(&w.adjc, &w.adjc_bytes, some(z.adjd * n), st));
-    SG_CKS(growT(&w.colors, &w.colors_bytes, some(V * n), st));
-    SG_CKS(growT(&w.partial, &w.partial_bytes, 8 * (V / 8 + 2) * n, st));
-    SG_CKS(growT(&w.root, &w.root_bytes, 8 * (size_t)std::max(g.V1, 1) * n, st));
-    SG_CKS(growT(&w.rticket, &w.rticket_bytes, 4 * kRootedTickets * n, st));
     SG_CKS(growT(&w.raw, &w.raw_bytes, 8 * (size_t)std::max(ncolorings, 1), st));
     SG_CKS(growT(&w.windows, &w.windows_bytes, 4 * 31 * (size_t)std::max(ncolorings, 1), st));
-    out.clear();
-    for (size_t i = 0; i < n; ++i)
-        out.push_back({(char *)w.arena + z.arena * i, (char *)w.agg + z.agg * i, (char *)w.cnt + z.cnt * i,
-                       (char *)w.scnt + z.scnt * i, w.adjc + z.adjd / 4 * i, w.colors + V * i,
-                       w.partial + (V / 8 + 2) * i, w.root + (size_t)std::max(g.V1, 1) * i, w.rticket + kRootedTickets * i});
+    out.assign(1, RootedSlot{});
+    Status first = rooted_grow(g, w, z, 0, out[0]);
+    if (first.code == 2) {   // the other slots' buffers serve nobody now
+        release_rooted(w, 1, st);
+        first = rooted_grow(g, w, z, 0, out[0]);
+    }
+    SG_CKS(first);
+    auto more = [](size_t need, size_t have) { return need > have ? need - have : 0; };
+    size_t taken = 0, room = 0;
+    int asked = 0;   // 1: the pool, 2: the driver too, whose answer can take milliseconds
+    for (int i = 1; i < want; ++i) {
+        const RootedBuffers b = rooted_buffers(w, i);
+        const size_t extra = more(z.tables(), *b.tables_bytes) + more(z.adjd, *b.adjd_bytes) + more(z.small, *b.small_bytes);
+        if (taken + extra > room && asked == 0) {
+            room = taken + pool_unused(g.device);
+            asked = 1;
+        }
+        if (taken + extra > room && asked == 1) {
+            size_t all = 0;
+            SG_CKS(available_bytes(g.device, all));
+            room = std::max(room, (size_t)((double)(taken + all) * share));
+            asked = 2;
+        }
+        if (taken + extra > room) break;
+        taken += extra;
+        RootedSlot s{};
+        const Status more_slots = rooted_grow(g, w, z, i, s);
+        if (more_slots.code == 2) {
+            release_rooted(w, i, st);
+            break;
+        }
+        SG_CKS(more_slots);
+        out.push_back(s);
+    }
     return Status::ok();
 }
 
@@ -1979,25 +2075,6 @@ Status make_streams(GraphState &gs, int n)
     return Status::ok();
 }
 
-// Slots for up to `want` colorings in flight that take no more than `share` of
-// the free memory.
-Status rooted_admit(const DeviceGraph &g, const Workspace &w, const RootedSizes &z, int want, double share, int &slots)
-{
-    slots = std::max(1, want);
-    if (slots == 1) return Status::ok();
-    // buffers that are there already need no answer from the driver
-    const size_t n = (size_t)slots;
-    if (w.arena_bytes >= z.arena * n && w.agg_bytes >= z.agg * n && w.cnt_bytes >= z.cnt * n && w.scnt_bytes >= z.scnt * n &&
-        w.adjc_bytes >= z.adjd * n && w.colors_bytes >= (size_t)g.V * n)
-        return Status::ok();
-    size_t free_b = 0, total_b = 0;
-    SG_CK(cudaMemGetInfo(&free_b, &total_b));
-    const size_t per = z.all() + (size_t)g.V + 8 * ((size_t)g.V / 8 + 2) + 8 * (size_t)g.V1;
-    const size_t have = w.arena_bytes + w.agg_bytes + w.cnt_bytes + w.scnt_bytes + w.adjc_bytes;
-    while (slots > 1 && per * (size_t)slots > (size_t)((double)(free_b + have) * share)) --slots;
-    return Status::ok();
-}
-
 Status count_rooted(RunCtx &c, const CountOptions &o, double *raw, CountStats *stats)
 {
     DeviceGraph &g = c.g;
@@ -2005,15 +2082,11 @@ Status count_rooted(RunCtx &c, const CountOptions &o, double *raw, CountStats *s
     cudaStream_t st = g.stream;
     const RootedSizes z = rooted_sizes(g, c.re->plan[c.fp64], g.V2, c.es);
     // several colorings in flight: the chains of one's hubs run beside the
-    // others' work (profiled launches one after another); a quarter of the
-    // memory at most, one coloring where more cannot be had
-    int S = 1;
+    // others' work (profiled launches one after another)
     const int most = o.batch > 0 ? std::min(o.batch, kRootedStreams) : kRootedStreams;
-    SG_CKS(rooted_admit(g, w, z, c.profile ? 1 : std::min(o.n_colorings, most), 0.25, S));
     std::vector<RootedSlot> slot;
-    Status room = rooted_reserve(g, w, z, S, o.n_colorings, slot);
-    if (room.code == 2 && S > 1) room = rooted_reserve(g, w, z, S = 1, o.n_colorings, slot);
-    SG_CKS(room);
+    SG_CKS(rooted_reserve(g, w, z, c.profile ? 1 : std::min(o.n_colorings, most), 0.25, o.n_colorings, slot));
+    const int S = (int)slot.size();
     std::vector<uint32_t> seeds(o.n_colorings);
     for (int i = 0; i < o.n_colorings; ++i) seeds[i] = o.seed_base + (uint32_t)i;
     SG_CKS(upload_seeds(g, w, seeds));
@@ -2045,7 +2118,7 @@ Status count_rooted(RunCtx &c, const CountOptions &o, double *raw, CountStats *s
     if (stats) {
         stats->device_ms = ms;
         stats->kernel_launches = c.launches;
-        stats->table_bytes = (int64_t)((z.arena + z.agg + z.cnt + z.scnt) * S);
+        stats->table_bytes = (int64_t)(z.tables() * S);
         stats->fused_launches = (int64_t)c.fused_ev.size();
         top_stage(c, stats);
         stats->fused_ms = ev_sum(c.fused_ev);
@@ -2133,8 +2206,8 @@ Status count_grouped(RunCtx &c, const CountOptions &o, double *raw, CountStats *
     cudaStream_t st = g.stream;
     int B = std::max(1, std::min(o.batch, o.n_colorings));
     {
-        size_t free_b = 0, total_b = 0;
-        SG_CK(cudaMemGetInfo(&free_b, &total_b));
+        size_t free_b = 0;
+        SG_CKS(available_bytes(g.device, free_b));
         const size_t V = (size_t)g.V;
         const size_t per = (size_t)p.arena_units * V * c.es + V + 8 * (V / 8 + 2);
         const size_t have = c.gs.ws.arena_bytes + c.gs.ws.colors_bytes + c.gs.ws.partial_bytes;
@@ -2196,6 +2269,7 @@ Status count(DeviceGraph &g, const Plan &p, const CountOptions &o, double *raw, 
         SG_CKS(rooted_entry(g, p, c.re));
         if (c.re->plan[c.fp64].ok) return count_rooted(c, o, raw, stats);
     }
+    release_rooted(gs.ws, 1, g.stream);   // room for the general path's tables
     SG_CKS(make_ctx_tables(g, p, gs, c.tab));
     c.exact = o.exact != 0;
     // hubs in exact order (the per-tile sums) on the plain and grouped forms;
@@ -2287,6 +2361,7 @@ static Status run_partial(DeviceGraph &g, const Plan &p, uint32_t seed, int mode
                           RunCtx &c, GraphState &gs)
 {
     if (g.V >= (1 << 28)) return Status{1, "counting supports graphs of fewer than 2^28 vertices"};
+    release_rooted(gs.ws, 1, g.stream);
     SG_CKS(make_ctx_tables(g, p, gs, c.tab));
     // the parity helpers run the reference's operation order; vertices above
     // hub_threshold go through the exact-order hub kernel
@@ -2333,7 +2408,7 @@ Status debug_sub_table(DeviceGraph &g, const Plan &p, uint32_t seed, int mode, i
         // every vertex's row (the counting calls leave out the rows nobody reads)
         const rt::RootedPlan &rp = c.re->plan[c.fp64];
         std::vector<RootedSlot> slot;
-        SG_CKS(rooted_reserve(g, gs.ws, rooted_sizes(g, rp, g.V1, c.es), 1, 1, slot));
+        SG_CKS(rooted_reserve(g, gs.ws, rooted_sizes(g, rp, g.V1, c.es), 1, 0.0, 1, slot));
         SG_CKS(upload_seeds(g, gs.ws, {seed}));
         SG_CKS(run_rooted(c, slot[0], g.V1, 0, nullptr, nullptr, s, g.stream));
         SG_CK(cudaStreamSynchronize(g.stream));
@@ -2390,7 +2465,7 @@ Status debug_root(DeviceGraph &g, const Plan &p, uint32_t seed, int mode, int hu
     if (mode == kModeReference || mode == kModeFP64) SG_CKS(rooted_entry(g, p, c.re));
     if (c.re && c.re->plan[c.fp64].ok) {
         std::vector<RootedSlot> slot;
-        SG_CKS(rooted_reserve(g, gs.ws, rooted_sizes(g, c.re->plan[c.fp64], g.V2, c.es), 1, 1, slot));
+        SG_CKS(rooted_reserve(g, gs.ws, rooted_sizes(g, c.re->plan[c.fp64], g.V2, c.es), 1, 0.0, 1, slot));
         SG_CKS(upload_seeds(g, gs.ws, {seed}));
         SG_CK(cudaMemsetAsync(gs.ws.root_vertex, 0, 8 * std::max<size_t>(1, (size_t)g.V), g.stream));
         SG_CKS(run_rooted(c, slot[0], g.V2, 0, gs.ws.raw, gs.ws.root_vertex, 0, g.stream));
@@ -2452,6 +2527,7 @@ Status count_jobs(DeviceGraph &g, const std::vector<const Plan *> &plans, const 
     const size_t V = (size_t)g.V;
     cudaStream_t st = g.stream;
     const Hubs hubs = plan_hubs(g, o.exact ? 0 : o.hub_threshold, false);
+    release_rooted(w, 1, st);
 
     // one context per job: its plan's device tables, its tables at arena_base
     std::vector<RunCtx> ctx;
@@ -2488,8 +2564,8 @@ Status count_jobs(DeviceGraph &g, const std::vector<const Plan *> &plans, const 
     int64_t launches = 0;
     for (int j0 = 0; j0 < n;) {
         // admission: jobs while their tables fit the free memory (at least one)
-        size_t free_b = 0, total_b = 0;
-        SG_CK(cudaMemGetInfo(&free_b, &total_b));
+        size_t free_b = 0;
+        SG_CKS(available_bytes(g.device, free_b));
         const size_t budget = (size_t)((double)(free_b + w.arena_bytes) * 0.85);
         size_t arena_sum = 0, hub_sum = 0;
         int j1 = j0;
@@ -2617,10 +2693,9 @@ static Status count_jobs_rooted(DeviceGraph &g, std::vector<RunCtx> &ctx, const 
     cudaStream_t st = g.stream;
     RootedSizes z;
     for (RunCtx &c : ctx) z.cover(rooted_sizes(g, c.re->plan[c.fp64], g.V2, c.es));
-    int S = 1;
-    SG_CKS(rooted_admit(g, w, z, std::min(o.batch > 0 ? o.batch : 8, n), 0.85, S));
     std::vector<RootedSlot> slot;
-    SG_CKS(rooted_reserve(g, w, z, S, n, slot));
+    SG_CKS(rooted_reserve(g, w, z, std::min(o.batch > 0 ? o.batch : 8, n), 0.85, n, slot));
+    const int S = (int)slot.size();
     SG_CKS(upload_seeds(g, w, std::vector<uint32_t>(seeds, seeds + n)));
     SG_CKS(make_streams(gs, S));
     std::vector<cudaEvent_t> ev_end(n, nullptr);
@@ -2655,7 +2730,7 @@ static Status count_jobs_rooted(DeviceGraph &g, std::vector<RunCtx> &ctx, const 
     if (stats) {
         stats->device_ms = total;
         stats->kernel_launches = launches;
-        stats->table_bytes = (int64_t)(z.all() * S);
+        stats->table_bytes = (int64_t)((z.tables() + z.adjd) * S);
     }
     return Status::ok();
 }
@@ -2699,6 +2774,7 @@ Status count_jobs_streams(DeviceGraph &g, const std::vector<const Plan *> &plans
         }
         if (all) return count_jobs_rooted(g, rc, seeds, o, raw, job_ms, stats);
     }
+    release_rooted(w, 1, st);
     const Hubs hubs = plan_hubs(g, o.hub_threshold, true);
     std::vector<RunCtx> ctx;
     ctx.reserve(n);
@@ -2726,8 +2802,8 @@ Status count_jobs_streams(DeviceGraph &g, const std::vector<const Plan *> &plans
     // colour-tagged adjacency, root partials and hub rows
     int S = std::max(1, std::min(o.batch > 0 ? o.batch : 8, n));
     {
-        size_t free_b = 0, total_b = 0;
-        SG_CK(cudaMemGetInfo(&free_b, &total_b));
+        size_t free_b = 0;
+        SG_CKS(available_bytes(g.device, free_b));
         const size_t per = max_arena + V + 8 * (V / 8 + 2) + hub_region + (adjc ? 4 * (size_t)g.nnz : 0);
         const size_t have = w.arena_bytes + w.hub_partial_bytes + w.adjc_bytes;
         while (S > 1 && per * (size_t)S > (size_t)((double)(free_b + have) * 0.85)) --S;
@@ -2754,11 +2830,7 @@ Status count_jobs_streams(DeviceGraph &g, const std::vector<const Plan *> &plans
         SG_CK(cudaMemcpyAsync(w.windows, win.data(), win.size() * 4, cudaMemcpyHostToDevice, st));
         SG_CK(cudaStreamSynchronize(st));
     }
-    while ((int)gs.streams.size() < S) {
-        cudaStream_t js;
-        SG_CK(cudaStreamCreateWithFlags(&js, cudaStreamNonBlocking));
-        gs.streams.push_back(js);
-    }
+    SG_CKS(make_streams(gs, S));
     for (RunCtx &c : ctx) {
         c.arena_per_coloring = max_arena;
         c.hub_pitch = hub_pitch;
