@@ -303,6 +303,46 @@ void release_rooted(Workspace &w, size_t first, cudaStream_t st)
     if (first < w.rooted.size()) w.rooted.resize(first);
 }
 
+// Streams for colorings and jobs in flight: a graph takes them on first use
+// and returns them, idle, when it is destroyed; a device keeps a few for the
+// next graph.
+constexpr size_t kIdleStreams = 16;
+std::map<int, std::vector<cudaStream_t>> g_idle_streams;   // per device, guarded by g_state_mu
+
+Status make_streams(const DeviceGraph &g, GraphState &gs, int n)
+{
+    {
+        std::lock_guard<std::mutex> lk(g_state_mu);
+        auto &idle = g_idle_streams[g.device];
+        while ((int)gs.streams.size() < n && !idle.empty()) {
+            gs.streams.push_back(idle.back());
+            idle.pop_back();
+        }
+    }
+    while ((int)gs.streams.size() < n) {
+        cudaStream_t js;
+        SG_CK(cudaStreamCreateWithFlags(&js, cudaStreamNonBlocking));
+        gs.streams.push_back(js);
+    }
+    return Status::ok();
+}
+
+void return_streams(int device, std::vector<cudaStream_t> &streams)
+{
+    for (cudaStream_t js : streams) {
+        cudaStreamSynchronize(js);
+        std::unique_lock<std::mutex> lk(g_state_mu);
+        auto &idle = g_idle_streams[device];
+        if (idle.size() < kIdleStreams) {
+            idle.push_back(js);
+        } else {
+            lk.unlock();
+            cudaStreamDestroy(js);
+        }
+    }
+    streams.clear();
+}
+
 // Register-blocked eMA tables of sub s: the output color sets (|s| colors out
 // of k) partitioned greedily into blocks U of |s|+1 colors, each block the
 // column ids of its held sets, streamed sets and outputs (-1: computed by
@@ -708,10 +748,7 @@ DeviceGraph::~DeviceGraph()
         if (p) cudaFreeAsync(p, stream);
     release_rooted(w, 0, stream);
     for (auto &kv : state.batches) free_batch(kv.second, stream);
-    for (cudaStream_t js : state.streams) {
-        cudaStreamSynchronize(js);
-        cudaStreamDestroy(js);
-    }
+    return_streams(device, state.streams);
     for (void *p : {(void *)d_off, (void *)d_adj, (void *)d_perm, (void *)d_iperm, (void *)d_jump, (void *)d_coef})
         if (p) cudaFreeAsync(p, stream);
     if (stream) {
@@ -2065,16 +2102,6 @@ void join_streams(GraphState &gs, int n, cudaStream_t st)
     }
 }
 
-Status make_streams(GraphState &gs, int n)
-{
-    while ((int)gs.streams.size() < n) {
-        cudaStream_t js;
-        SG_CK(cudaStreamCreateWithFlags(&js, cudaStreamNonBlocking));
-        gs.streams.push_back(js);
-    }
-    return Status::ok();
-}
-
 Status count_rooted(RunCtx &c, const CountOptions &o, double *raw, CountStats *stats)
 {
     DeviceGraph &g = c.g;
@@ -2090,7 +2117,7 @@ Status count_rooted(RunCtx &c, const CountOptions &o, double *raw, CountStats *s
     std::vector<uint32_t> seeds(o.n_colorings);
     for (int i = 0; i < o.n_colorings; ++i) seeds[i] = o.seed_base + (uint32_t)i;
     SG_CKS(upload_seeds(g, w, seeds));
-    if (S > 1) SG_CKS(make_streams(c.gs, S));
+    if (S > 1) SG_CKS(make_streams(g, c.gs, S));
     cudaEvent_t e0, e1;
     SG_CK(cudaEventCreate(&e0));
     SG_CK(cudaEventCreate(&e1));
@@ -2697,7 +2724,7 @@ static Status count_jobs_rooted(DeviceGraph &g, std::vector<RunCtx> &ctx, const 
     SG_CKS(rooted_reserve(g, w, z, std::min(o.batch > 0 ? o.batch : 8, n), 0.85, n, slot));
     const int S = (int)slot.size();
     SG_CKS(upload_seeds(g, w, std::vector<uint32_t>(seeds, seeds + n)));
-    SG_CKS(make_streams(gs, S));
+    SG_CKS(make_streams(g, gs, S));
     std::vector<cudaEvent_t> ev_end(n, nullptr);
     cudaEvent_t ev0;
     SG_CK(cudaEventCreate(&ev0));
@@ -2830,7 +2857,7 @@ Status count_jobs_streams(DeviceGraph &g, const std::vector<const Plan *> &plans
         SG_CK(cudaMemcpyAsync(w.windows, win.data(), win.size() * 4, cudaMemcpyHostToDevice, st));
         SG_CK(cudaStreamSynchronize(st));
     }
-    SG_CKS(make_streams(gs, S));
+    SG_CKS(make_streams(g, gs, S));
     for (RunCtx &c : ctx) {
         c.arena_per_coloring = max_arena;
         c.hub_pitch = hub_pitch;
