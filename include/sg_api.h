@@ -250,7 +250,10 @@ sg_status sg_estimate(const double *raw, int32_t n, int32_t k, int32_t automorph
  * original vertex order. */
 sg_status sg_colors(sg_graph g, int32_t k, uint32_t seed, int32_t *colors);
 /* the count table of sub s after one coloring (DataTableColMajor columns,
- * column-major [L][V], original order; float or double by mode) */
+ * column-major [L][V], original order; float or double by mode).  Both table
+ * helpers compute in the reference's operation order: with hub_threshold 0 in
+ * the default form, with hub_threshold > 0 on the general path, whose hub
+ * kernel takes the vertices of more neighbours. */
 sg_status sg_debug_sub_table(sg_graph g, sg_plan p, uint32_t seed, int32_t mode, int32_t hub_threshold,
                              int32_t s, void *out);
 /* per-vertex root values (bufLastSub, CountMat.cpp:815-831) and their sum */

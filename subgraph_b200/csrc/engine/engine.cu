@@ -2430,7 +2430,8 @@ Status debug_sub_table(DeviceGraph &g, const Plan &p, uint32_t seed, int mode, i
         return Status::ok();
     }
     c.exact = true;   // the reference's operation order
-    if (mode == kModeReference || mode == kModeFP64) SG_CKS(rooted_entry(g, p, c.re));
+    // a hub threshold selects the general path, whose hubs it names
+    if (hub_threshold <= 0 && (mode == kModeReference || mode == kModeFP64)) SG_CKS(rooted_entry(g, p, c.re));
     if (c.re && c.re->plan[c.fp64].ok) {
         // every vertex's row (the counting calls leave out the rows nobody reads)
         const rt::RootedPlan &rp = c.re->plan[c.fp64];
@@ -2489,7 +2490,8 @@ Status debug_root(DeviceGraph &g, const Plan &p, uint32_t seed, int mode, int hu
     SG_CKS(growT(&gs.ws.root_vertex, &gs.ws.root_vertex_bytes, 8 * std::max<size_t>(1, (size_t)g.V), g.stream));
     if (g.V >= (1 << 28)) return Status{1, "counting supports graphs of fewer than 2^28 vertices"};
     c.exact = true;   // the reference's operation order
-    if (mode == kModeReference || mode == kModeFP64) SG_CKS(rooted_entry(g, p, c.re));
+    // a hub threshold selects the general path, whose hubs it names
+    if (hub_threshold <= 0 && (mode == kModeReference || mode == kModeFP64)) SG_CKS(rooted_entry(g, p, c.re));
     if (c.re && c.re->plan[c.fp64].ok) {
         std::vector<RootedSlot> slot;
         SG_CKS(rooted_reserve(g, gs.ws, rooted_sizes(g, c.re->plan[c.fp64], g.V2, c.es), 1, 0.0, 1, slot));
