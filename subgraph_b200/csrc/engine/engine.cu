@@ -2,6 +2,7 @@
 #include "engine.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -274,7 +275,7 @@ Status available_bytes(int device, size_t &bytes)
     return Status::ok();
 }
 
-uint64_t g_grow_count = 0;   // re-allocations so far (the workspace generation)
+std::atomic<uint64_t> g_grow_count{0};   // re-allocations so far, of every thread (the workspace generation)
 
 Status grow(void **p, size_t *have, size_t need, cudaStream_t st)
 {
