@@ -232,7 +232,7 @@ sg_status sg_count(sg_graph g, sg_plan p, const sg_count_opts *o, double *raw, s
  * the jobs run as persistent work-queue launches instead (all their
  * sub-template stages in one queue, waves admitted by free device memory).
  * From opts also: mode, hub_threshold, exact, wait_limit_ms, no_autotune,
- * no_blocked.  job_ms (optional, n_jobs): each job's latency from the start of
+ * no_blocked, no_rooted, no_flat.  job_ms (optional, n_jobs): each job's latency from the start of
  * the call's launches (stream form) or of its wave's launch (persistent form)
  * to the end of its last stage.  The reference
  * runs one template per CountMat::compute (CountMat.cpp:79-266); this is the

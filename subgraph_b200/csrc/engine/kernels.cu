@@ -73,9 +73,9 @@ void launch_color(const ColorArgs &a, int ncolorings, cudaStream_t st)
 // the original order (which fixes the summation order) with ids mapped
 // through perm.  A block takes kRemapPer consecutive entries of the new
 // adjacency: a list of tens of thousands of entries on one warp took 0.4 ms
-// of an upload of 4 M entries, the even split takes 56 us.  The vertex of a
-// thread's entry is found by bisection of the new offsets, once a thread and
-// then by stepping.
+// of an upload of 4 M entries, the even split takes 56 us.  The vertices of the
+// block's first and last entries are found by bisection of the new offsets,
+// those of the entries between by bisection between the two.
 // ---------------------------------------------------------------------------
 constexpr int kRemapThreads = 256, kRemapEach = 8, kRemapPer = kRemapThreads * kRemapEach;
 

@@ -159,7 +159,7 @@ struct RootedTables {
     std::vector<const int32_t *> blk;
     std::vector<int32_t> blk_shape, blk_nblocks;
 };
-// Fills host images; `bytes` is what upload_rooted_tables copies.
+// Builds the tables of a plan and copies them to the device.
 cudaError_t upload_rooted_tables(const Plan &p, const RootedPlan &rp, RootedTables &t, cudaStream_t st);
 
 // blocks of an index structure (engine.cu): the register-blocked schedule

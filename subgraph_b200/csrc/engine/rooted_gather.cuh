@@ -30,7 +30,7 @@ __device__ __forceinline__ bool chunk_of(const ChunkMap &m, int t, int &v0, int 
 // without its own color, in list order.  Three parts:
 //   hubs    a CTA per (vertex, columns), the longest lists first;
 //   wide    a warp per run of vertices, R sums a lane, rows staged in shared
-//           memory by bulk copies;
+//           memory by 16-byte asynchronous copies (cp.async);
 //   narrow  G lanes a vertex, R sums a lane, rows read where they lie.
 // One kernel takes the hubs first and then the wide or the narrow part, so
 // that the longest chains run beside the other vertices.
