@@ -884,7 +884,8 @@ void release_plan_tables(uint64_t uid)
         }
         if (prev < 0) cudaGetDevice(&prev);
         cudaSetDevice(it->first.first);
-        cudaFree(it->second.tab.mem);
+        // calls that read them have returned, after their work was done
+        if (it->second.tab.mem) cudaFreeAsync(it->second.tab.mem, cudaStreamLegacy);
         it = g_rooted.erase(it);
     }
     if (prev >= 0) cudaSetDevice(prev);
@@ -1787,13 +1788,13 @@ Status rooted_entry(DeviceGraph &g, const Plan &p, const RootedEntry *&out)
     if (e.plan[0].ok || e.plan[1].ok) {
         const cudaError_t ce = rt::upload_rooted_tables(p, e.plan[0], e.tab, g.stream);
         if (ce != cudaSuccess) {
-            cudaFree(e.tab.mem);
+            if (e.tab.mem) cudaFreeAsync(e.tab.mem, g.stream);
             return Status{ce == cudaErrorMemoryAllocation ? 2 : 3, std::string("rooted tables: ") + cudaGetErrorString(ce)};
         }
     }
     std::lock_guard<std::mutex> lk(g_state_mu);
     auto ins = g_rooted.try_emplace(key, std::move(e));
-    if (!ins.second) cudaFree(e.tab.mem);   // another thread made them first
+    if (!ins.second && e.tab.mem) cudaFreeAsync(e.tab.mem, g.stream);   // another thread made them first
     out = &ins.first->second;
     return Status::ok();
 }

@@ -242,7 +242,7 @@ cudaError_t upload_rooted_tables(const Plan &p, const RootedPlan &rp, RootedTabl
         if (q.s != 0 && rooted_blocks(k - 1, q.n - 1, q.pm - 1, rows, t.blk_nblocks[i], t.blk_shape[i]))
             blk[i] = put(rows.data(), rows.size() * 4);
     }
-    cudaError_t e = cudaMalloc(&t.mem, std::max<size_t>(img.size(), 16));
+    cudaError_t e = cudaMallocAsync(&t.mem, std::max<size_t>(img.size(), 16), st);
     if (e != cudaSuccess) return e;
     if (!img.empty()) {
         // pageable source: the call returns once it has been read

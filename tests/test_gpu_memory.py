@@ -91,3 +91,19 @@ def test_first_call_on_a_new_graph_is_a_warm_one():
             ms.append(time.perf_counter() - t0)
         del g
     assert sorted(first)[12] <= sorted(warm)[37] + 1.5e-4, (sorted(first)[12], sorted(warm)[37])
+
+
+def test_first_call_with_a_new_template():
+    """A template made, counted and dropped per call: its tables' memory comes from
+    the pool (P3, R-MAT scale 16: 0.5 ms and up to 4.5 above the second call's
+    0.1 with the driver's own allocations, 0.06 on full-width tables)."""
+    g = sg.DeviceGraph.from_rmat(16, 16, seed=2)
+    first, warm = [], []
+    for _ in range(41):
+        t = sg.Graph(*TEMPLATES["p3"])
+        for ms in (first, warm):
+            t0 = time.perf_counter()
+            sg.count(g, t, 1, 5)
+            ms.append((time.perf_counter() - t0) * 1e3)
+        del t
+    assert sorted(first)[20] <= sorted(warm)[20] + 0.25, (sorted(first)[20], sorted(warm)[20])
