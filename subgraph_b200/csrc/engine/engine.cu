@@ -897,8 +897,11 @@ Status graph_create(const int32_t *offsets, const int32_t *neighbors, int32_t V,
     if (V < 0 || nnz < 0 || nnz > 0x7fffffffLL) return Status{1, "vertex or entry count out of range"};
     if (!offsets || (nnz > 0 && !neighbors)) return Status{1, "null graph array"};
     if (offsets[0] != 0 || offsets[V] != nnz) return Status{1, "offsets[0] must be 0 and offsets[V] must equal nnz"};
-    for (int32_t v = 0; v < V; ++v)
-        if (offsets[v + 1] < offsets[v]) return Status{1, "offsets are not monotone"};
+    // no way out of the loop, so that it is vectorised: 39 us at 2^18 vertices (95 or
+    // 190 with one, by where the compiler happened to place it)
+    int32_t falls = 0;
+    for (int32_t v = 0; v < V; ++v) falls |= offsets[v + 1] < offsets[v];
+    if (falls) return Status{1, "offsets are not monotone"};
     // neighbour ids are range-checked by the remap kernel (graph_finish)
     std::unique_ptr<DeviceGraph> g;
     SG_CKS(new_device_graph(device, V, nnz, g));
