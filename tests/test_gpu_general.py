@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 import subgraph_b200 as sg
+from oracle import oracle as O
 from subgraph_b200._lib import CountOpts, check
 from tests.helpers import TEMPLATES, prufer_tree, rel
 from tests.test_gpu_parity import dev_graph, sha
@@ -107,3 +108,27 @@ def test_overflowing_counts_are_infinite_in_every_form():
         for form in [{}, dict(batch=1)] + FORMS:
             raw = sg.count(g, t, 1, 3, exact=True, autotune=False, **form)[0]
             assert raw == np.inf, (edges, form, raw)
+
+
+def test_template_that_only_the_general_path_takes(golden):
+    """15 vertices, a path of 14 with a leaf at its eighth: a step of 6 and 2
+    vertices whose rooted rows (3003 + 14 + 3432 columns, eight vertices a tile) do
+    not fit shared memory where the general path's (5005 + 105 and a part of the
+    outputs) do.  Plain, tuned and in groups, and jobs beside one that the default
+    form would take."""
+    g, col, row = dev_graph(golden, "rmat10")
+    edges = [(i, i + 1) for i in range(13)] + [(7, 14)]
+    t = sg.Graph(15, edges)
+    P = O.Plan(15, edges)
+    want = [O.count_coloring(col, row, P, O.colors(9 + i, len(col) - 1, 15)) for i in range(2)]
+    raw, st = sg.count(g, t, 2, 9, exact=True, autotune=False, return_stats=True)
+    assert all(rel(a, b) <= 1e-12 for a, b in zip(raw, want)), (raw, want)
+    off, st2 = sg.count(g, t, 2, 9, exact=True, autotune=False, flat=False, return_stats=True)
+    assert st["table_bytes"] == st2["table_bytes"] and np.array_equal(raw, off)
+    for kw in (dict(autotune=True), dict(batch=2), dict(hub_threshold=16, autotune=False)):
+        got = sg.count(g, t, 2, 9, exact=True, **kw)
+        assert all(rel(a, b) <= 1e-12 for a, b in zip(got, want)), (kw, got, want)
+    t5 = sg.Graph(*TEMPLATES["tree5"])
+    got = sg.count_jobs(g, [t, t5, t], [9, 4, 10], exact=True)
+    for a, b in zip(got, [want[0], sg.count(g, t5, 1, 4, exact=True)[0], want[1]]):
+        assert rel(a, b) <= 1e-12, (got, want)
