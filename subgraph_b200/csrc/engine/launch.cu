@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -22,8 +23,19 @@ std::map<std::pair<int, const void *>, Kernel> g_kernels;   // per (device, kern
 
 int resident_ctas(const void *kern, int threads, size_t smem)
 {
+    // this thread's last answers: what they rest on, a raised limit and the
+    // occupancy of a size, does not change (the lock and the maps cost a call of
+    // seven launches 1 us)
+    struct Answer {
+        const void *kern;
+        size_t smem;
+        int dev, threads, n;
+    };
+    thread_local Answer answers[64];
     int dev = 0;
     cudaGetDevice(&dev);
+    Answer &mine = answers[((uintptr_t)kern >> 4 ^ smem >> 4 ^ (size_t)dev) & 63];
+    if (mine.kern == kern && mine.smem == smem && mine.threads == threads && mine.dev == dev) return mine.n;
     std::lock_guard<std::mutex> lk(g_mu);
     Kernel &k = g_kernels[{dev, kern}];
     if (!k.raised) {
@@ -35,11 +47,15 @@ int resident_ctas(const void *kern, int threads, size_t smem)
                        cudaSuccess;
     }
     auto it = k.ctas.find({threads, smem});
-    if (it != k.ctas.end()) return it->second;
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess) return 1;
-    if (k.ctas.size() >= 64) k.ctas.clear();
-    return k.ctas[{threads, smem}] = std::max(n, 1);
+    int n = it != k.ctas.end() ? it->second : 0;
+    if (n == 0) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess) return 1;
+        n = std::max(n, 1);
+        if (k.ctas.size() >= 64) k.ctas.clear();
+        k.ctas[{threads, smem}] = n;
+    }
+    if (k.raised) mine = {kern, smem, dev, threads, n};
+    return n;
 }
 
 }  // namespace sg
