@@ -1811,9 +1811,8 @@ struct RootedSlot {
     int32_t *ticket;
 };
 constexpr int kRootedStreams = 4;
-// counters of a step: the column blocks' chunks, the hub items last; a slot
-// has them for every step of a template (at most 15)
-constexpr int kStepTickets = 64, kRootedTickets = 16 * kStepTickets;
+// a slot has the counters of every step of a template (at most 15)
+constexpr int kRootedTickets = 16 * rt::kStepTickets;
 
 // Per-slot bytes of a plan whose tables have `rows` rows.
 struct RootedSizes {
@@ -1943,6 +1942,30 @@ int hub_deg(const DeviceGraph &g, int nA, int slots)
     return (int)std::min<int64_t>(8192, std::max<int64_t>(256, d));
 }
 
+// The vertices [0, hubs) a gather takes as hubs.  Wide rows: none where they would
+// hold more than three quarters of the entries: then the hubs are the graph, and a
+// warp a vertex is faster (2000 vertices all joined, paths of 10 and 13: 2.64 ->
+// 1.48 and 24.3 -> 7.7 ms; of 7 vertices, narrow rows, 0.31 -> 0.54).
+int32_t gather_hubs(const DeviceGraph &g, int32_t V, int nA, int slots)
+{
+    const int32_t hubs = std::min(V, degree_prefix(g, hub_deg(g, nA, slots) + 1));
+    if (nA <= 64 || (int64_t)hubs * g.max_degree <= g.nnz / 4 * 3) return hubs;
+    int64_t left = g.nnz / 4 * 3;
+    for (int32_t v = 0; v < hubs; ++v)
+        if ((left -= g.h_degree[v]) < 0) return 0;
+    return hubs;
+}
+
+// Where the hub items go one to an SM (hub_turn): no more of them than SMs, and the
+// longest list outlasting the other work by far (19 cycles a neighbour against
+// about 25 an entry over 148 SMs: even at 1/110 of the entries).  20 lists of
+// 100,000 among 200,000 vertices (1/40 each), 7-spider: 3.08 -> 1.53 ms; on R-MAT
+// graphs, whose longest list has 1/75 of the entries and less, it cost 2 to 4 %.
+bool hubs_spread(const DeviceGraph &g, const rt::GatherArgs &a)
+{
+    return (int64_t)g.max_degree * 50 > g.nnz && (int64_t)a.hubs * ((a.nA + 31) / 32) <= g.sm_count;
+}
+
 // One coloring (window `coloring`) on stream st: tables of `rows` rows, the
 // steps of the subs >= upto, with the root step its raw count.
 Status run_rooted(RunCtx &c, const RootedSlot &w, int32_t rows, int coloring, double *raw_out, double *root_vertex, int upto,
@@ -1978,7 +2001,7 @@ Status run_rooted(RunCtx &c, const RootedSlot &w, int32_t rows, int coloring, do
     rt::launch_edges(ea, std::max(ea.hubs, degree_prefix(g, 32)), c.fp64, st);
     c.launches += 2;
     SG_CK(cudaGetLastError());
-    SG_CK(cudaMemsetAsync(w.ticket, 0, 4 * kStepTickets * rp.steps.size(), st));
+    SG_CK(cudaMemsetAsync(w.ticket, 0, 4 * rt::kStepTickets * rp.steps.size(), st));
     int root_n = 0;
     for (size_t i = 0; i < rp.steps.size(); ++i) {
         const rt::Step &q = rp.steps[i];
@@ -2010,15 +2033,17 @@ Status run_rooted(RunCtx &c, const RootedSlot &w, int32_t rows, int coloring, do
             if (root && q.main_leaf) ga.out = w.agg, ga.out_pitch = 1;
             else if (q.main_leaf) ga.out = const_cast<void *>(rooted_table(c, rp, w, rows, q.s)), ga.out_pitch = rp.tab[q.s].pitch;
             else ga.out = w.agg, ga.out_pitch = rp.agg_pitch;
-            ga.hubs = std::min(V, degree_prefix(g, hub_deg(g, q.nA, co.slots) + 1));
+            ga.hubs = gather_hubs(g, V, q.nA, co.slots);
             // a warp's chunk: 512 entries, fewer where the graph would not give every
             // warp of the device four of them (0.8 M entries: 236 CTAs of 740)
             const int entries = (int)std::min<int64_t>(512, std::max<int64_t>(64, g.nnz / (g.sm_count * 128)));
             // (a warp to a vertex of a long list: k_gather's rule)
             ga.map = rt::make_chunks(g.h_degree, ga.hubs, V, entries, 32 / rt::gather_lanes(ga),
                                      ga.slots <= 1 ? 32 : ga.slots <= 4 ? 128 : 1 << 30, 32);
-            ga.ticket = w.ticket + kStepTickets * i;
-            ga.hub_ticket = ga.ticket + kStepTickets - 1;
+            ga.ticket = w.ticket + rt::kStepTickets * i;
+            ga.sm_seen = (uint32_t *)(ga.ticket + rt::kColumnBlocks);
+            ga.spread = hubs_spread(g, ga);
+            ga.hub_ticket = ga.ticket + rt::kStepTickets - 1;
             c.launches += rt::launch_gather(ga, c.fp64, g.sm_count, st);
             agg = ga.out;
             agg_pitch = ga.out_pitch;

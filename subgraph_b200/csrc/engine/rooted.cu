@@ -100,7 +100,8 @@ void launch_edges(const EdgeArgs &a, int32_t mid, bool fp64, cudaStream_t st)
 bool gather_fits(int k, int nA, int nR, bool fp64)
 {
     // row offsets in 16 bits (13 beside a slot's member), a counter per column block
-    return k <= 16 && nR < 0x1fff && (size_t)nR * (fp64 ? 8 : 4) + 32 < 0xffff && nA <= 32 * 256;
+    // (of 128 slots at least; more than 128 columns, the narrower ones take one)
+    return k <= 16 && nR < 0x1fff && (size_t)nR * (fp64 ? 8 : 4) + 32 < 0xffff && nA <= 128 * kColumnBlocks;
 }
 
 int gather_lanes(const GatherArgs &a) { return a.slots <= 1 ? 1 : a.slots <= 4 ? 4 : a.slots <= 8 ? 8 : a.slots <= 16 ? 16 : 32; }

@@ -85,7 +85,11 @@ struct GatherArgs {
     const uint16_t *idx;                // [k-1][nA] column of the neighbour's row, 0xffff: adds nothing
     ChunkMap map;                       // of the vertices [hubs, V)
     int32_t *ticket, *hub_ticket;       // zeroed: a chunk counter per column block; the hub items' counter
+    uint32_t *sm_seen;                  // zeroed: a bit per SM that has a CTA [kSmWords]
+    int32_t spread;                     // hub items: one CTA of an SM takes them
 };
+// counters of a step: column blocks (at most kColumnBlocks), SMs, hub items
+constexpr int kColumnBlocks = 56, kSmWords = 7, kStepTickets = kColumnBlocks + kSmWords + 1;
 
 struct EmaArgs {
     int32_t k, V, nA, nM, nO, S;        // columns of aggregate, main and result rows; splits per result
