@@ -255,25 +255,40 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_wide(GatherArgs a)
     for (int i = threadIdx.x; i < NP * 32; i += kGatherThreads) (&need[0][0])[i] = 0;
     for (int i = threadIdx.x; i < MB * R * 32; i += kGatherThreads) (&member[0][0])[i] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < a.k * 32 * N; i += kGatherThreads) {
-        const int d = i / (32 * N), c = i / 256 % NC, l = i / 8 % 32, r = c * 8 + i % 8;
-        const int slot = slot0 + r * 32 + l;
-        uint16_t x = 0xffffu;
-        if (d > 0 && r < R)
+    // four entries a thread at a time, their loads in flight together: on a graph of
+    // a hundred vertices the tables are the kernel's time
+    for (int i0 = threadIdx.x; i0 < a.k * 32 * N; i0 += 4 * kGatherThreads) {
+        uint16_t y[4][M];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * kGatherThreads, d = i / (32 * N), l = i / 8 % 32, r = i / 256 % NC * 8 + i % 8;
+            const int slot = slot0 + r * 32 + l;
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+                y[u][m] = d > 0 && d < a.k && r < R && slot < a.start[m + 1] - a.start[m]
+                              ? __ldg(a.idx + (size_t)(d - 1) * a.nA + a.start[m] + slot)
+                              : (uint16_t)0xffffu;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * kGatherThreads;
+            if (i >= a.k * 32 * N) break;
+            const int d = i / (32 * N), l = i / 8 % 32, r = i / 256 % NC * 8 + i % 8;
+            uint16_t x = 0xffffu;
+#pragma unroll
             for (int m = 0; m < M; ++m) {
-                if (slot >= a.start[m + 1] - a.start[m]) break;
-                const uint16_t y = __ldg(a.idx + (size_t)(d - 1) * a.nA + a.start[m] + slot);
-                if (y == 0xffffu) continue;
-                x = y;
+                if (y[u][m] == 0xffffu) continue;
+                x = y[u][m];
                 if (MB == 1 && m == 1) atomicOr(&member[r][l], 1u << d);
                 if (MB > 1) atomicOr(&member[r * MB + m][l], 1u << d);
             }
-        if (x != 0xffffu) {   // whole sectors: the two pieces of 32 bytes
-            const int q = x / PE & ~1;
-            atomicOr(&need[q >> 5][q & 31], 1u << d);
-            if ((uint32_t)(q + 1) * 16 < row_bytes) atomicOr(&need[q >> 5][(q & 31) + 1], 1u << d);
+            if (x != 0xffffu) {   // whole sectors: the two pieces of 32 bytes
+                const int q = x / PE & ~1;
+                atomicOr(&need[q >> 5][q & 31], 1u << d);
+                if ((uint32_t)(q + 1) * 16 < row_bytes) atomicOr(&need[q >> 5][(q & 31) + 1], 1u << d);
+            }
+            tab[i] = (uint16_t)(x == 0xffffu ? row_bytes : (uint32_t)x * (uint32_t)sizeof(T));
         }
-        tab[i] = (uint16_t)(x == 0xffffu ? row_bytes : (uint32_t)x * (uint32_t)sizeof(T));
     }
     if (blockIdx.y == 0) hub_part<T, 32>(a, ring_raw, s_turn);
     __syncthreads();
