@@ -1998,7 +1998,8 @@ Status run_rooted(RunCtx &c, const RootedSlot &w, int32_t rows, int coloring, do
     ea.cnt = w.cnt;
     ea.scnt = rp.need_scaled ? w.scnt : nullptr;
     ea.cnt_pitch = rp.cnt_pitch;
-    rt::launch_edges(ea, std::max(ea.hubs, degree_prefix(g, 32)), c.fp64, st);
+    const int32_t mid = std::max(ea.hubs, degree_prefix(g, 32));
+    rt::launch_edges(ea, mid, std::max(mid, degree_prefix(g, 9)), c.fp64, st);
     c.launches += 2;
     SG_CK(cudaGetLastError());
     SG_CK(cudaMemsetAsync(w.ticket, 0, 4 * rt::kStepTickets * rp.steps.size(), st));

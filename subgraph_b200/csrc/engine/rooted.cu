@@ -19,7 +19,9 @@ constexpr int kEdgeThreads = 256;
 // Per coloring: every neighbour entry's color relative to its vertex, and the
 // vertex's neighbour count of each relative color (the rows of a
 // sub-template of two vertices, exact integers in any order).  A block's
-// threads take one hub, or 8 vertices at a warp each, or 32 at 8 threads each.
+// threads take one hub, or 8 vertices at a warp each, 32 at 8 threads each, or
+// 128 of at most eight neighbours at 2 threads each (8 threads of which most had
+// nothing to do took 62 us at 10^6 vertices of degree 4).
 // ---------------------------------------------------------------------------
 template <typename T, int G>
 __device__ __forceinline__ void edge_rows(const EdgeArgs &a, int v, int t, unsigned *cnt)
@@ -42,21 +44,40 @@ __device__ __forceinline__ void edge_rows(const EdgeArgs &a, int v, int t, unsig
     }
 }
 
+// 16 bytes a thread: rows are whole pieces of 16
 template <typename T> __device__ __forceinline__ void count_row(const EdgeArgs &a, int v, int t, int G, const unsigned *cnt)
 {
-    for (int j = t; j < a.cnt_pitch; j += G) {
-        const T x = j < a.k - 1 ? (T)cnt[j + 1] : T(0);
-        reinterpret_cast<T *>(a.cnt)[(size_t)v * a.cnt_pitch + j] = x;
-        if (a.scnt) reinterpret_cast<T *>(a.scnt)[(size_t)v * a.cnt_pitch + j] = leaf_value(x, true);
+    constexpr int E = 16 / (int)sizeof(T);
+    for (int j = t * E; j < a.cnt_pitch; j += G * E) {
+        __align__(16) T x[E], y[E];
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            x[i] = j + i < a.k - 1 ? (T)cnt[j + i + 1] : T(0);
+            y[i] = leaf_value(x[i], true);
+        }
+        *reinterpret_cast<uint4 *>(reinterpret_cast<T *>(a.cnt) + (size_t)v * a.cnt_pitch + j) = *reinterpret_cast<uint4 *>(x);
+        if (a.scnt)
+            *reinterpret_cast<uint4 *>(reinterpret_cast<T *>(a.scnt) + (size_t)v * a.cnt_pitch + j) = *reinterpret_cast<uint4 *>(y);
     }
 }
 
-template <typename T> __global__ void __launch_bounds__(kEdgeThreads) k_edges(EdgeArgs a, int mid, int nb_mid)
+// G threads a vertex, the block's vertices from v0
+template <typename T, int G>
+__device__ __forceinline__ void edge_group(const EdgeArgs &a, int v0, int end, unsigned *cnt_s)
 {
-    __shared__ unsigned cnt_s[32 * 17];
-    for (int i = threadIdx.x; i < 32 * 17; i += kEdgeThreads) cnt_s[i] = 0;
+    const int g = threadIdx.x / G, t = threadIdx.x % G, v = v0 + g;
+    if (v < end) edge_rows<T, G>(a, v, t, cnt_s + g * 17);
+    __syncwarp();
+    if (v < end) count_row<T>(a, v, t, G, cnt_s + g * 17);
+}
+
+template <typename T> __global__ void __launch_bounds__(kEdgeThreads) k_edges(EdgeArgs a, int mid, int low, int nb_mid, int nb_8)
+{
+    __shared__ unsigned cnt_s[kEdgeThreads / 2 * 17];
+    int blk = blockIdx.x;
+    const int rows = blk < a.hubs + nb_mid ? kEdgeThreads / 32 : blk < a.hubs + nb_mid + nb_8 ? kEdgeThreads / 8 : kEdgeThreads / 2;
+    for (int i = threadIdx.x; i < rows * 17; i += kEdgeThreads) cnt_s[i] = 0;
     __syncthreads();
-    const int blk = blockIdx.x;
     if (blk < a.hubs) {
         // counters of a warp each, then their sum
         unsigned *mine = cnt_s + (threadIdx.x >> 5) * 17;
@@ -71,30 +92,22 @@ template <typename T> __global__ void __launch_bounds__(kEdgeThreads) k_edges(Ed
         count_row<T>(a, blk, threadIdx.x, kEdgeThreads, cnt_s);
         return;
     }
-    if (blk < a.hubs + nb_mid) {
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int v = a.hubs + (blk - a.hubs) * (kEdgeThreads / 32) + w;
-        if (v >= mid) return;
-        edge_rows<T, 32>(a, v, lane, cnt_s + w * 17);
-        __syncwarp();
-        count_row<T>(a, v, lane, 32, cnt_s + w * 17);
-        return;
-    }
-    const int g = threadIdx.x >> 3, t = threadIdx.x & 7;
-    const int v = mid + (blk - a.hubs - nb_mid) * (kEdgeThreads / 8) + g;
-    if (v < a.V1) edge_rows<T, 8>(a, v, t, cnt_s + g * 17);
-    __syncwarp();
-    if (v < a.V1) count_row<T>(a, v, t, 8, cnt_s + g * 17);
+    blk -= a.hubs;
+    if (blk < nb_mid) return edge_group<T, 32>(a, a.hubs + blk * (kEdgeThreads / 32), mid, cnt_s);
+    blk -= nb_mid;
+    if (blk < nb_8) return edge_group<T, 8>(a, mid + blk * (kEdgeThreads / 8), low, cnt_s);
+    edge_group<T, 2>(a, low + (blk - nb_8) * (kEdgeThreads / 2), a.V1, cnt_s);
 }
 
-void launch_edges(const EdgeArgs &a, int32_t mid, bool fp64, cudaStream_t st)
+void launch_edges(const EdgeArgs &a, int32_t mid, int32_t low, bool fp64, cudaStream_t st)
 {
     if (a.V1 <= 0) return;
     const int nb_mid = (mid - a.hubs + kEdgeThreads / 32 - 1) / (kEdgeThreads / 32);
-    const int nb_low = (a.V1 - mid + kEdgeThreads / 8 - 1) / (kEdgeThreads / 8);
-    const int grid = a.hubs + nb_mid + nb_low;
-    if (fp64) k_edges<double><<<grid, kEdgeThreads, 0, st>>>(a, mid, nb_mid);
-    else k_edges<float><<<grid, kEdgeThreads, 0, st>>>(a, mid, nb_mid);
+    const int nb_8 = (low - mid + kEdgeThreads / 8 - 1) / (kEdgeThreads / 8);
+    const int nb_2 = (a.V1 - low + kEdgeThreads / 2 - 1) / (kEdgeThreads / 2);
+    const int grid = a.hubs + nb_mid + nb_8 + nb_2;
+    if (fp64) k_edges<double><<<grid, kEdgeThreads, 0, st>>>(a, mid, low, nb_mid, nb_8);
+    else k_edges<float><<<grid, kEdgeThreads, 0, st>>>(a, mid, low, nb_mid, nb_8);
 }
 
 bool gather_fits(int k, int nA, int nR, bool fp64)

@@ -114,8 +114,8 @@ struct RootArgs {
     double *root_partial, *root_vertex; // per tile, per vertex (optional)
 };
 
-// vertices [hubs, mid) a warp each, [mid, V1) 8 threads each
-void launch_edges(const EdgeArgs &a, int32_t mid, bool fp64, cudaStream_t st);
+// vertices [hubs, mid) a warp each, [mid, low) 8 threads each, [low, V1) 2
+void launch_edges(const EdgeArgs &a, int32_t mid, int32_t low, bool fp64, cudaStream_t st);
 // false: the shapes do not fit the kernels (the caller takes the general path)
 bool gather_fits(int k, int nA, int nR, bool fp64);
 int gather_lanes(const GatherArgs &a);  // threads a vertex
