@@ -71,7 +71,7 @@ __device__ __forceinline__ bool hub_turn(const GatherArgs &a)
     return !(atomicOr(a.sm_seen + (sm >> 5), bit) & bit);
 }
 
-template <typename T, int GH> __device__ __forceinline__ void hub_part(const GatherArgs &a, unsigned char *smem, const int &s_turn)
+template <typename T, int GH> __device__ __forceinline__ void hub_part(const GatherArgs &a, unsigned char *smem)
 {
     constexpr int NPF = 32 / GH, PER = hub_fills<GH>(); // neighbours a fill, fills
     constexpr int NPW = PER * NPF;                  // neighbours a producer and batch
@@ -87,7 +87,7 @@ template <typename T, int GH> __device__ __forceinline__ void hub_part(const Gat
     const uint32_t row_bytes = (uint32_t)a.pitch * (uint32_t)sizeof(T);
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) s_item = s_turn ? atomicAdd(a.hub_ticket, 1) : 0x7fffffff;
+        if (threadIdx.x == 0) s_item = atomicAdd(a.hub_ticket, 1);
         __syncthreads();
         const int v = s_item / nblk, col0 = (s_item - v * nblk) * GH;
         if (v >= a.hubs) break;
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_wide(GatherArgs a)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t row_bytes = ((uint32_t)a.nR * (uint32_t)sizeof(T) + 15u) / 16u * 16u, rs = wide_stride(row_bytes);
     const int slot0 = blockIdx.y * (32 * R);
-    __shared__ int s_turn;   // thread 0's own
+    __shared__ int s_turn;
     if (threadIdx.x == 0 && blockIdx.y == 0) s_turn = hub_turn(a);
     for (int i = threadIdx.x; i < NP * 32; i += kGatherThreads) (&need[0][0])[i] = 0;
     for (int i = threadIdx.x; i < MB * R * 32; i += kGatherThreads) (&member[0][0])[i] = 0;
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_wide(GatherArgs a)
             tab[i] = (uint16_t)(x == 0xffffu ? row_bytes : (uint32_t)x * (uint32_t)sizeof(T));
         }
     }
-    if (blockIdx.y == 0) hub_part<T, 32>(a, ring_raw, s_turn);
+    if (blockIdx.y == 0 && s_turn) hub_part<T, 32>(a, ring_raw);
     __syncthreads();
     for (int i = threadIdx.x; i < kWarps * RR; i += kGatherThreads)
         *reinterpret_cast<uint4 *>(ring_raw + (size_t)i * rs + row_bytes) = make_uint4(0, 0, 0, 0);
@@ -459,7 +459,7 @@ template <typename T, int G, int R, int M, int U, int GH> __global__ void __laun
     __shared__ uint32_t hits[R][G], seconds[R][G];            // a bit per color: some set holds it; the second does
     uint16_t *tab = reinterpret_cast<uint16_t *>(smem_raw);   // [k][G][N]
     const int slot0 = blockIdx.y * (G * R);
-    __shared__ int s_turn;   // thread 0's own
+    __shared__ int s_turn;
     if (threadIdx.x == 0 && blockIdx.y == 0) s_turn = hub_turn(a);
     for (int i = threadIdx.x; i < R * G; i += kGatherThreads) (&hits[0][0])[i] = (&seconds[0][0])[i] = 0;
     __syncthreads();
@@ -479,7 +479,7 @@ template <typename T, int G, int R, int M, int U, int GH> __global__ void __laun
         tab[i] = x;
     }
     unsigned char *rest = smem_raw + ((size_t)a.k * G * N * 2 + 15) / 16 * 16;
-    if (blockIdx.y == 0) hub_part<T, GH>(a, rest, s_turn);
+    if (blockIdx.y == 0 && s_turn) hub_part<T, GH>(a, rest);
     __syncthreads();
     T *sacc = reinterpret_cast<T *>(rest) + threadIdx.x;   // M > 2: [R][M][threads], a thread's own
     const int lane = threadIdx.x & 31, lg = lane % G, grp = lane / G;
