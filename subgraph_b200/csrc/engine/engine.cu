@@ -1999,7 +1999,13 @@ Status run_rooted(RunCtx &c, const RootedSlot &w, int32_t rows, int coloring, do
     ea.scnt = rp.need_scaled ? w.scnt : nullptr;
     ea.cnt_pitch = rp.cnt_pitch;
     const int32_t mid = std::max(ea.hubs, degree_prefix(g, 32));
-    rt::launch_edges(ea, mid, std::max(mid, degree_prefix(g, 9)), c.fp64, st);
+    // vertices of at most eight neighbours: two threads each where eight would be
+    // more threads than the device holds at once (a single edge on uniform graphs:
+    // 25,000 vertices 23.5 us with eight, 23.9 with two; 50,000 25.6 and 25.0;
+    // 200,000 33.7 and 30.1)
+    const int32_t low = std::max(mid, degree_prefix(g, 9));
+    const bool two = (int64_t)(g.V1 - low) * 8 > (int64_t)g.sm_count * 2048;
+    rt::launch_edges(ea, mid, two ? low : g.V1, c.fp64, st);
     c.launches += 2;
     SG_CK(cudaGetLastError());
     SG_CK(cudaMemsetAsync(w.ticket, 0, 4 * rt::kStepTickets * rp.steps.size(), st));

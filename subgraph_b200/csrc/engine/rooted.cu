@@ -44,10 +44,12 @@ __device__ __forceinline__ void edge_rows(const EdgeArgs &a, int v, int t, unsig
     }
 }
 
-// 16 bytes a thread: rows are whole pieces of 16
-template <typename T> __device__ __forceinline__ void count_row(const EdgeArgs &a, int v, int t, int G, const unsigned *cnt)
+// A vertex's row by its G threads, an element each; by two threads in pieces of 16
+// bytes, of which rows are whole ones.  (Pieces by eight threads leave most of
+// them idle: the kernel 14.2 us against 13.4, P3 on R-MAT scale 16.)
+template <typename T, int G> __device__ __forceinline__ void count_row(const EdgeArgs &a, int v, int t, const unsigned *cnt)
 {
-    constexpr int E = 16 / (int)sizeof(T);
+    constexpr int E = G == 2 ? 16 / (int)sizeof(T) : 1;
     for (int j = t * E; j < a.cnt_pitch; j += G * E) {
         __align__(16) T x[E], y[E];
 #pragma unroll
@@ -55,9 +57,15 @@ template <typename T> __device__ __forceinline__ void count_row(const EdgeArgs &
             x[i] = j + i < a.k - 1 ? (T)cnt[j + i + 1] : T(0);
             y[i] = leaf_value(x[i], true);
         }
-        *reinterpret_cast<uint4 *>(reinterpret_cast<T *>(a.cnt) + (size_t)v * a.cnt_pitch + j) = *reinterpret_cast<uint4 *>(x);
-        if (a.scnt)
-            *reinterpret_cast<uint4 *>(reinterpret_cast<T *>(a.scnt) + (size_t)v * a.cnt_pitch + j) = *reinterpret_cast<uint4 *>(y);
+        T *o = reinterpret_cast<T *>(a.cnt) + (size_t)v * a.cnt_pitch + j;
+        T *so = reinterpret_cast<T *>(a.scnt) + (size_t)v * a.cnt_pitch + j;
+        if constexpr (E == 1) {
+            *o = x[0];
+            if (a.scnt) *so = y[0];
+        } else {
+            *reinterpret_cast<uint4 *>(o) = *reinterpret_cast<uint4 *>(x);
+            if (a.scnt) *reinterpret_cast<uint4 *>(so) = *reinterpret_cast<uint4 *>(y);
+        }
     }
 }
 
@@ -68,12 +76,12 @@ __device__ __forceinline__ void edge_group(const EdgeArgs &a, int v0, int end, u
     const int g = threadIdx.x / G, t = threadIdx.x % G, v = v0 + g;
     if (v < end) edge_rows<T, G>(a, v, t, cnt_s + g * 17);
     __syncwarp();
-    if (v < end) count_row<T>(a, v, t, G, cnt_s + g * 17);
+    if (v < end) count_row<T, G>(a, v, t, cnt_s + g * 17);
 }
 
 template <typename T> __global__ void __launch_bounds__(kEdgeThreads) k_edges(EdgeArgs a, int mid, int low, int nb_mid, int nb_8)
 {
-    __shared__ unsigned cnt_s[kEdgeThreads / 2 * 17];
+    extern __shared__ unsigned cnt_s[];   // [most vertices of a block][17]
     int blk = blockIdx.x;
     const int rows = blk < a.hubs + nb_mid ? kEdgeThreads / 32 : blk < a.hubs + nb_mid + nb_8 ? kEdgeThreads / 8 : kEdgeThreads / 2;
     for (int i = threadIdx.x; i < rows * 17; i += kEdgeThreads) cnt_s[i] = 0;
@@ -89,7 +97,7 @@ template <typename T> __global__ void __launch_bounds__(kEdgeThreads) k_edges(Ed
             cnt_s[threadIdx.x] = s;
         }
         __syncthreads();
-        count_row<T>(a, blk, threadIdx.x, kEdgeThreads, cnt_s);
+        count_row<T, kEdgeThreads>(a, blk, threadIdx.x, cnt_s);
         return;
     }
     blk -= a.hubs;
@@ -106,8 +114,11 @@ void launch_edges(const EdgeArgs &a, int32_t mid, int32_t low, bool fp64, cudaSt
     const int nb_8 = (low - mid + kEdgeThreads / 8 - 1) / (kEdgeThreads / 8);
     const int nb_2 = (a.V1 - low + kEdgeThreads / 2 - 1) / (kEdgeThreads / 2);
     const int grid = a.hubs + nb_mid + nb_8 + nb_2;
-    if (fp64) k_edges<double><<<grid, kEdgeThreads, 0, st>>>(a, mid, low, nb_mid, nb_8);
-    else k_edges<float><<<grid, kEdgeThreads, 0, st>>>(a, mid, low, nb_mid, nb_8);
+    // a block's counters (below the 48 KB any kernel may have); what an SM's blocks
+    // do not take is cache for the colors
+    const size_t smem = (size_t)kEdgeThreads / (nb_2 > 0 ? 2 : 8) * 17 * sizeof(unsigned);
+    if (fp64) k_edges<double><<<grid, kEdgeThreads, smem, st>>>(a, mid, low, nb_mid, nb_8);
+    else k_edges<float><<<grid, kEdgeThreads, smem, st>>>(a, mid, low, nb_mid, nb_8);
 }
 
 bool gather_fits(int k, int nA, int nR, bool fp64)

@@ -53,6 +53,22 @@ def test_counts_equal_general_path(graph):
             assert (k > 5 or np.all(a > 0)) and all(rel(x, y) <= 1e-12 for x, y in zip(a, b)), (k, edges, kw, a, b)
 
 
+@pytest.mark.parametrize("ring", [37880, 37888, 37889, 60001])
+def test_many_vertices_of_few_neighbours(ring):
+    """More of them than SMs x 256 (37,888 on 148) take two threads each; their lists
+    have one to eight entries, beside longer ones."""
+    rng = np.random.default_rng(ring)
+    e = [(i, (i + 1) % ring) for i in range(ring)]
+    e += [(int(v), (int(v) + j) % ring) for v in rng.integers(0, ring, ring // 8) for j in range(2, 2 + int(v) % 4)]
+    e += [(ring, i) for i in range(0, 3000, 2)] + [(ring + 1, i) for i in range(20)] + [(0, ring + 2)]
+    g = _csc(ring + 4, e).device_graph()
+    for k, edges in [(k, [(i, i + 1) for i in range(k - 1)]) for k in (2, 3, 5, 9)] + [TEMPLATES["star4"], TEMPLATES["spider7"]]:
+        t = sg.Graph(k, edges)
+        for kw in (dict(exact=True), dict(mode=sg.MODE_FP64)):
+            a, b = _both(g, t, 1, 3 + k, autotune=False, **kw)
+            assert a[0] > 0 and rel(a[0], b[0]) <= 1e-12, (k, edges, kw, a, b)
+
+
 def _edges(V, src, dst):
     return sg.DeviceGraph.from_edges(V, src.astype(np.int32), dst.astype(np.int32))
 
